@@ -387,8 +387,8 @@ class RichardsonLucyBatch:
         return list(out)
 
     def launch_config(self):
-        """(CTAs per SM, queue order, grouping) of the persistent launch: order 0 = largest
-        images first, 1 = grouped by PSF width; grouping 0-3 = the work items' shapes (tiles per
+        """(CTAs per SM, queue order, grouping) of the persistent launch: order 0 = one
+        queue, largest images first, 1 = a queue per PSF width; grouping 0-3 = the work items' shapes (tiles per
         item by PSF width, see ``tile_widths``)."""
         bps, order, group = ctypes.c_int32(0), ctypes.c_int32(0), ctypes.c_int32(0)
         check(lib().iane_gb_rl_batch_config(self._batch, ctypes.byref(bps), ctypes.byref(order),

@@ -98,8 +98,8 @@ bool work_layout(const DevView& v, long long pitch)
 int tiles_of(int n) { return (n + kBatchTile - 1) / kBatchTile; }
 
 // Queue orders of one phase's items (the autotuner picks one per batch).
-constexpr int kOrderLargestFirst = 0; // images by descending tile count
-constexpr int kOrderByWidth = 1;      // images by PSF width, then by descending tile count
+constexpr int kOrderLargestFirst = 0; // one queue, images by descending tile count
+constexpr int kOrderByWidth = 1;      // a queue per PSF width, images by descending tile count
 constexpr int kOrders = 2;
 
 // Item shapes: tiles per item (along x) by PSF width, one rule per grouping level. Narrow PSFs
@@ -135,6 +135,64 @@ std::vector<BatchItem> make_items(const std::vector<int>& nx, const std::vector<
 		}
 	}
 	return items;
+}
+
+// What a 64x64 tile of a kx x ky PSF costs: its taps plus kTileOverhead, what staging, hand-off
+// and the epilogue take beside them.
+constexpr float kTileOverhead = 60.0f;
+float tile_cost(int kx, int ky) { return static_cast<float>(kx) * static_cast<float>(ky) + kTileOverhead; }
+
+// The queues of make_items' list: one for the whole batch, or one per PSF width with the SMs
+// shared out in proportion to the widths' work (at least one SM each, largest remainders).
+BatchQueues make_queues(const std::vector<BatchItem>& items, const std::vector<int>& kx, const std::vector<int>& ky,
+	int order, int sms)
+{
+	BatchQueues q{};
+	q.sms = std::max(1, std::min(sms, kBatchSmTable));
+	double work[kBatchClasses] = {}, all = 0.0;
+	for (size_t i = 0; i < items.size(); ++i) {
+		const int image = items[i].image;
+		const bool next = i == 0 || (order == kOrderByWidth && kx[image] != kx[items[i - 1].image]);
+		if (next) q.of[q.classes++] = BatchClass{static_cast<int>(i), 0, 0.0f};
+		++q.of[q.classes - 1].count;
+		const double c = static_cast<double>(items[i].count) * tile_cost(kx[image], ky[image]);
+		work[q.classes - 1] += c;
+		all += c;
+	}
+	// as many SMs as the share gives, rounded by largest remainder; a queue whose share is
+	// below one SM still gets one while there are SMs for every queue
+	std::vector<int> sm(q.classes, 0);
+	int left = q.sms;
+	for (int c = 0; c < q.classes; ++c) {
+		q.of[c].cost = static_cast<float>(work[c] / q.of[c].count);
+		sm[c] = std::max(1, static_cast<int>(work[c] / all * q.sms));
+		left -= sm[c];
+	}
+	auto short_of = [&](int c) { return work[c] / all * q.sms - sm[c]; };
+	for (; left > 0 && q.classes > 0; --left) {
+		int best = 0;
+		for (int c = 1; c < q.classes; ++c)
+			if (short_of(c) > short_of(best)) best = c;
+		++sm[best];
+	}
+	for (; left < 0; ++left) {
+		int best = -1;
+		for (int c = 0; c < q.classes; ++c)
+			if (sm[c] > 0 && (best < 0 || sm[c] > sm[best])) best = c;
+		if (best < 0) break;
+		--sm[best];
+	}
+	int at = 0;
+	for (int c = 0; c < q.classes; ++c)
+		for (int k = 0; k < sm[c] && at < q.sms; ++k) q.start[at++] = static_cast<unsigned char>(c);
+	return q;
+}
+
+// CTAs per SM of a launch that is not tuned: no more than one phase has items for.
+int default_blocks_per_sm(size_t items, int most, int sms)
+{
+	const long long want = (static_cast<long long>(items) + sms - 1) / sms;
+	return static_cast<int>(std::max(1LL, std::min<long long>(most, want)));
 }
 
 // ---------------------------------------------------------------------------------------
@@ -285,10 +343,10 @@ int fill_images(const iane_gb_rl_batch* b, const DevView* obs, const DevView* es
 BatchSync sync_words(const iane_gb_rl_batch* b, char* base)
 {
 	unsigned int* words = reinterpret_cast<unsigned int*>(base + b->sync_off);
-	return BatchSync{words, reinterpret_cast<int*>(words + 1), words + 2};
+	return BatchSync{words, reinterpret_cast<int*>(words + kBatchClasses), words + kBatchClasses + 1};
 }
 
-size_t sync_bytes(int count) { return static_cast<size_t>(count + 2) * sizeof(unsigned int); }
+size_t sync_bytes(int count) { return static_cast<size_t>(count + kBatchClasses + 1) * sizeof(unsigned int); }
 
 // Build descriptors for one run and the graph that performs it: clear the queue, abort flag
 // and completion counters, the start values, then the one persistent launch.
@@ -326,8 +384,9 @@ int build_graph(iane_gb_rl_batch* b, const DevView* obs, const DevView* est, int
 	}
 	batch_init_kernel<<<dim3(n, 16), 256, 0, s0>>>(b->d_init, starts, eps, init);
 	if (iterations > 0) {
-		st = launch_batch_persistent(b->d_images, b->d_items, static_cast<int>(b->items.size()), 2 * iterations, sync,
-			status, b->blocks_per_sm * device_sm_count(), b->smem, s0);
+		const BatchQueues queues = make_queues(b->items, b->kx, b->ky, b->order, device_sm_count());
+		st = launch_batch_persistent(b->d_images, b->d_items, queues, 2 * iterations, sync, status,
+			b->blocks_per_sm * device_sm_count(), b->smem, s0);
 		if (st) return abort_capture(st);
 	} else {
 		batch_init_kernel<<<dim3(n, 16), 256, 0, s0>>>(b->d_init, starts, eps, -1);
@@ -428,14 +487,14 @@ int autotune(iane_gb_rl_batch* b, cudaStream_t stream)
 		if (cudaMemcpy(d_items, items.data(), items.size() * sizeof(BatchItem), cudaMemcpyHostToDevice) != cudaSuccess) {
 			return cuda_fail(cudaGetLastError(), "autotune: upload items");
 		}
+		const BatchQueues queues = make_queues(items, b->kx, b->ky, order, sms);
 		ms = 0.0f;
 		for (int rep = 0; rep < 3; ++rep) {
 			if (cudaMemsetAsync(sync.queue, 0, sync_bytes(n), stream) != cudaSuccess) {
 				return cuda_fail(cudaGetLastError(), "autotune: clear queue");
 			}
 			cudaEventRecord(t0, stream);
-			const int s = launch_batch_persistent(d_images, d_items, static_cast<int>(items.size()), 4, sync, status,
-				bps * sms, b->smem, stream);
+			const int s = launch_batch_persistent(d_images, d_items, queues, 4, sync, status, bps * sms, b->smem, stream);
 			if (s) return s;
 			cudaEventRecord(t1, stream);
 			IANE_GB_CUDA(cudaEventSynchronize(t1), "autotune: time");
@@ -541,10 +600,10 @@ int iane_gb_rl_batch_prepare(const iane_gb_view* psfs, int count, const int32_t*
 	b->sync_off = off;
 	off += align_up(sync_bytes(count));
 	b->scratch_bytes = off + kAlignB;
-	b->blocks_per_sm = batch_blocks_per_sm(b->smem);
-	b->order = kOrderLargestFirst;
+	b->order = kOrderByWidth;
 	b->group = 0;
 	b->items = make_items(b->nx, b->ny, b->kx, b->order, b->group);
+	b->blocks_per_sm = default_blocks_per_sm(b->items.size(), batch_blocks_per_sm(b->smem), device_sm_count());
 	if (cudaMalloc(&b->d_items, b->items.size() * sizeof(BatchItem)) != cudaSuccess ||
 	    cudaMalloc(&b->d_images, count * sizeof(BatchImage)) != cudaSuccess ||
 	    cudaMalloc(&b->d_init, count * sizeof(InitDesc)) != cudaSuccess ||

@@ -5,7 +5,8 @@
 // repeated once per phase (phase 2t = pass A of iteration t, 2t + 1 = pass B); item k is
 // (phase k / T, entry k % T) for T items per pass. CTAs (a few per SM) take items from an
 // atomic counter in queue order and run the tiled FP32 convolution body with that image's TMA
-// map, PSF and fused epilogue. RL's only dependency is per image: a phase of an image reads
+// map, PSF and fused epilogue. The images of one PSF width can have a queue of their own
+// (BatchClass): the CTAs of an SM then stay on one width's code until its queue is empty. RL's only dependency is per image: a phase of an image reads
 // (with a halo) what the image's previous phase wrote and overwrites what it read, so an item
 // of phase p waits until all tiles of its image's phase p - 1 are done -- a per-image
 // completion counter that reaches p * tiles -- instead of a grid-wide drain between passes.
@@ -52,8 +53,28 @@ struct BatchItem {
 	int image_tiles; // the image's 64x64 tiles (its completions per phase), read at hand-off
 };
 
-// Device words of a run, cleared before the launch: the queue counter, the abort flag and one
-// completion counter per image.
+// Queues of one launch: at most one per PSF width (odd, 1 .. 31).
+constexpr int kBatchClasses = 16;
+constexpr int kBatchSmTable = 512;
+
+// One queue: items first .. first + count - 1 of a phase, taken phases times over, and what one
+// of them costs on average (any unit).
+struct BatchClass {
+	int first;
+	int count;
+	float cost;
+};
+
+// The queues of a launch and which of them the CTAs of each SM start on.
+struct BatchQueues {
+	int classes;
+	int sms;
+	BatchClass of[kBatchClasses];
+	unsigned char start[kBatchSmTable]; // by SM id, modulo sms
+};
+
+// Device words of a run, cleared before the launch: one counter per queue, the abort flag and
+// one completion counter per image.
 struct BatchSync {
 	unsigned int* queue;
 	int* abort;
@@ -61,8 +82,8 @@ struct BatchSync {
 };
 
 // The persistent launch (rl_batch_kernel.cu): `grid` CTAs of 128 threads, `smem` bytes of
-// dynamic shared memory (batch_tile_smem over the batch), items * phases work items.
-int launch_batch_persistent(const BatchImage* images, const BatchItem* items, int items_per_phase, int phases,
+// dynamic shared memory (batch_tile_smem over the batch).
+int launch_batch_persistent(const BatchImage* images, const BatchItem* items, const BatchQueues& queues, int phases,
 	BatchSync sync, int* status, int grid, size_t smem, cudaStream_t stream);
 
 // Dynamic shared memory a tile of PSF width kx, height ky needs.

@@ -314,7 +314,7 @@ int iane_gb_wiener_destroy(iane_gb_wiener_plan* plan);
  * dependency and completion work over several tiles).
  * psfs: `count` f32 2-D device views (odd extents up to 31 x 63); extents: 2*count ints
  * (nx, ny per image). IANE_GB_BATCH_AUTOTUNE times the launch's CTAs per SM, its queue order
- * (largest images first, or grouped by PSF width) and the work items' shapes (the grouping level:
+ * (largest images first, or a queue per PSF width) and the work items' shapes (the grouping level:
  * 0 one tile per item; 1 two tiles for PSFs up to 11 wide; 2 four tiles for PSFs up to 11 wide;
  * 3 four tiles up to 7 wide and two up to 15) on this batch and caches the choice per (image
  * shapes, PSF sizes, dtype, SM count) in the file named by the environment variable
@@ -328,8 +328,8 @@ int iane_gb_rl_batch_prepare(const iane_gb_view* psfs, int count, const int32_t*
 size_t iane_gb_rl_batch_scratch_bytes(const iane_gb_rl_batch* batch);
 /* Width of every image's work items: 64 x the tiles per item (their height is 64). */
 int iane_gb_rl_batch_tiles(const iane_gb_rl_batch* batch, int32_t* tile_width);
-/* The persistent launch's CTAs per SM, queue order (0: largest images first, 1: by PSF width)
- * and grouping level of the work items. */
+/* The persistent launch's CTAs per SM, queue order (0: one queue, largest images first; 1: a
+ * queue per PSF width, the default) and grouping level of the work items. */
 int iane_gb_rl_batch_config(const iane_gb_rl_batch* batch, int32_t* blocks_per_sm, int32_t* order,
 	int32_t* grouping);
 /* Pin the launch configuration (for example one tuned offline): CTAs per SM from 1 to the
