@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(128) cnn_tc_conv_kernel(const __grid_constant_
 			} else {
 				tma_load_5d(st, &map1, 0, x0 - 1, y0 - 1, z0 - 1, 2 * (p - a.steps0), &full[p % S]);
 			}
-			tc::bulk_load(st + AB, a.packed + static_cast<size_t>(p) * (b_bytes(N) / 2), b_bytes(N), &full[p % S]);
+			bulk_copy_shared(st + AB, a.packed + static_cast<size_t>(p) * (b_bytes(N) / 2), b_bytes(N), &full[p % S]);
 		};
 		bool ok = true;
 		for (int p = 0; p < S && p < a.steps; ++p) load(p);

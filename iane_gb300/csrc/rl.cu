@@ -874,6 +874,7 @@ int iane_gb_rl_run(iane_gb_rl_plan* plan, const iane_gb_view* observed, const ia
 	ea.obs = obs.ptr;
 	for (int i = 0; i < 3; ++i) ea.os[i] = obs.stride[i];
 	ea.obs_u8 = obs.dtype == IANE_GB_U8;
+	ea.obs_rows = obs.dtype == IANE_GB_F32 && obs.stride[0] == 4;
 	ea.eps = epsilon;
 	ea.nx = nx;
 	ea.ny = ny;
@@ -1135,6 +1136,7 @@ int iane_gb_rl_run_noalloc(const iane_gb_view* psf, const iane_gb_view* observed
 	ea.obs = obs.ptr;
 	for (int i = 0; i < 3; ++i) ea.os[i] = obs.stride[i];
 	ea.obs_u8 = obs.dtype == IANE_GB_U8;
+	ea.obs_rows = obs.dtype == IANE_GB_F32 && obs.stride[0] == 4;
 	ea.eps = epsilon;
 	ea.nx = nx;
 	ea.ny = ny;

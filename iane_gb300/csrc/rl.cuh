@@ -23,6 +23,7 @@ struct EpiRatio {
 	const char* obs;    // observed view (u8 or f32, any strides)
 	long long os[3];
 	int obs_u8;
+	int obs_rows;       // f32 with packed rows: a lane's row segment is one pointer and its offsets
 	float eps;
 	int nx, ny;
 
@@ -40,10 +41,21 @@ struct EpiRatio {
 			return;
 		}
 		float r[N];
+		if (obs_rows && xo + N <= nx) {
+			const float* o = reinterpret_cast<const float*>(obs + y * os[1] + z * os[2]) + xo;
 #pragma unroll
-		for (int i = 0; i < N; ++i) {
-			const float p = v[i];
-			r[i] = xo + i < nx ? observed(xo + i, y, z) / (p > eps ? p : eps) : 0.0f;
+			for (int i = 0; i < N; ++i) r[i] = o[i];
+#pragma unroll
+			for (int i = 0; i < N; ++i) {
+				const float p = v[i];
+				r[i] = r[i] / (p > eps ? p : eps);
+			}
+		} else {
+#pragma unroll
+			for (int i = 0; i < N; ++i) {
+				const float p = v[i];
+				r[i] = xo + i < nx ? observed(xo + i, y, z) / (p > eps ? p : eps) : 0.0f;
+			}
 		}
 		float* out = ratio + z * plane + y * pitch + xo;
 		if (xo + N <= nx) {

@@ -23,70 +23,108 @@ constexpr size_t kAlignB = 256;
 constexpr int kMaxBatchIterations = 4096;
 inline size_t align_up(size_t v) { return (v + kAlignB - 1) / kAlignB * kAlignB; }
 
+// Blocks that share one image in the start-value kernels.
+constexpr int kStartBlocks = 32;
+
 // Per-image description for the batched start-value kernels.
 struct InitDesc {
 	DevView obs;
 	DevView est;
 	float* work;
+	double* parts;   // kStartBlocks partial sums, in the ratio image (256 bytes or more), which is
+	                 // not in use before the first pass
 	long long pitch;
 	int in_place;
 };
 
-__global__ void batch_mean_kernel(const InitDesc* d, float* starts, float eps)
+// Sums of the observed images in FP64: block (i, j) takes rows j, j + kStartBlocks, .. of image
+// i, a warp per row. (One block per image, with an index division per pixel, took 2.6 ms on the
+// largest images of a 256-image batch.)
+__global__ void __launch_bounds__(256) batch_mean_kernel(const InitDesc* d)
 {
 	const InitDesc& im = d[blockIdx.x];
 	const int nx = im.obs.ext[0], ny = im.obs.ext[1];
-	const long long n = static_cast<long long>(nx) * ny;
+	if (nx == 0 || ny == 0) return; // no ratio image to hold the partial sums
+	const bool u8 = im.obs.dtype == IANE_GB_U8;
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	double s = 0.0;
-	for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-		const int x = static_cast<int>(i % nx), y = static_cast<int>(i / nx);
-		const char* p = im.obs.ptr + x * im.obs.stride[0] + y * im.obs.stride[1];
-		s += im.obs.dtype == IANE_GB_U8 ? static_cast<double>(*reinterpret_cast<const uint8_t*>(p))
-			: static_cast<double>(*reinterpret_cast<const float*>(p));
+	for (int y = blockIdx.y + kStartBlocks * warp; y < ny; y += kStartBlocks * 8) {
+		const char* row = im.obs.ptr + y * im.obs.stride[1];
+#pragma unroll 4
+		for (int x = lane; x < nx; x += 32) {
+			const char* p = row + x * im.obs.stride[0];
+			s += u8 ? static_cast<double>(*reinterpret_cast<const uint8_t*>(p))
+				: static_cast<double>(*reinterpret_cast<const float*>(p));
+		}
 	}
-	__shared__ double red[32];
+	__shared__ double red[8];
 	for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-	if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+	if (lane == 0) red[warp] = s;
 	__syncthreads();
 	if (threadIdx.x == 0) {
 		double t = 0.0;
-		for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) t += red[w];
-		const float mean = static_cast<float>(t / static_cast<double>(n > 0 ? n : 1));
-		starts[blockIdx.x] = mean > eps ? mean : eps;
+		for (int w = 0; w < 8; ++w) t += red[w];
+		im.parts[blockIdx.y] = t;
 	}
 }
 
-// mode: RL start mode, or -1 = copy the work estimate out to the caller's view.
-__global__ void batch_init_kernel(const InitDesc* d, const float* starts, float eps, int mode)
+// A plan's packed PSF and adjoint in rows of `pitch` taps, zero beyond kx.
+__global__ void batch_taps_kernel(const float* psf, const float* adj, int kx, int ky, int pitch, float* out)
+{
+	const int n = pitch * ky;
+	for (int i = threadIdx.x; i < 2 * n; i += blockDim.x) {
+		const int j = i < n ? i : i - n;
+		const int x = j % pitch, y = j / pitch;
+		out[i] = x < kx ? (i < n ? psf : adj)[y * kx + x] : 0.0f;
+	}
+}
+
+// mode: RL start mode, or -1 = copy the work estimate out to the caller's view. Block (i, j) takes
+// rows j, j + kStartBlocks, .. of image i, a warp per row.
+__global__ void __launch_bounds__(256) batch_init_kernel(const InitDesc* d, float eps, int mode)
 {
 	const InitDesc& im = d[blockIdx.x];
 	const int nx = im.obs.ext[0], ny = im.obs.ext[1];
-	const long long n = static_cast<long long>(nx) * ny;
-	for (long long i = blockIdx.y * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-	     i += static_cast<long long>(gridDim.y) * blockDim.x) {
-		const int x = static_cast<int>(i % nx), y = static_cast<int>(i / nx);
-		float& w = im.work[y * im.pitch + x];
-		char* e = im.est.ptr + x * im.est.stride[0] + y * im.est.stride[1];
-		if (mode < 0) {
-			if (!im.in_place) {
-				if (im.est.dtype == IANE_GB_U8) {
-					*reinterpret_cast<uint8_t*>(e) = to_gray8(w);
-				} else {
-					*reinterpret_cast<float*>(e) = w;
+	if (nx == 0 || ny == 0) return;
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	float flat = 0.0f;
+	if (mode == IANE_GB_RL_INIT_MEAN) {
+		// the partial sums in the same order in every warp
+		double t = im.parts[lane];
+		for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+		const long long n = static_cast<long long>(nx) * ny;
+		const float mean = static_cast<float>(t / static_cast<double>(n > 0 ? n : 1));
+		flat = mean > eps ? mean : eps;
+	}
+	for (int y = blockIdx.y + kStartBlocks * warp; y < ny; y += kStartBlocks * 8) {
+		float* work = im.work + y * im.pitch;
+		char* est = im.est.ptr + y * im.est.stride[1];
+		const char* obs = im.obs.ptr + y * im.obs.stride[1];
+		for (int x = lane; x < nx; x += 32) {
+			float& w = work[x];
+			char* e = est + x * im.est.stride[0];
+			if (mode < 0) {
+				if (!im.in_place) {
+					if (im.est.dtype == IANE_GB_U8) {
+						*reinterpret_cast<uint8_t*>(e) = to_gray8(w);
+					} else {
+						*reinterpret_cast<float*>(e) = w;
+					}
 				}
+			} else if (mode == IANE_GB_RL_INIT_GIVEN) {
+				if (!im.in_place) w = *reinterpret_cast<const float*>(e);
+			} else if (mode == IANE_GB_RL_INIT_MEAN) {
+				w = flat;
+			} else {
+				const char* p = obs + x * im.obs.stride[0];
+				const float o = im.obs.dtype == IANE_GB_U8 ? static_cast<float>(*reinterpret_cast<const uint8_t*>(p))
+					: *reinterpret_cast<const float*>(p);
+				w = o > eps ? o : eps;
 			}
-		} else if (mode == IANE_GB_RL_INIT_GIVEN) {
-			if (!im.in_place) w = *reinterpret_cast<const float*>(e);
-		} else if (mode == IANE_GB_RL_INIT_MEAN) {
-			w = starts[blockIdx.x];
-		} else {
-			const char* p = im.obs.ptr + x * im.obs.stride[0] + y * im.obs.stride[1];
-			const float o = im.obs.dtype == IANE_GB_U8 ? static_cast<float>(*reinterpret_cast<const uint8_t*>(p))
-				: *reinterpret_cast<const float*>(p);
-			w = o > eps ? o : eps;
 		}
 	}
 }
+static_assert(kStartBlocks == 32, "one partial sum per lane");
 
 bool work_layout(const DevView& v, long long pitch)
 {
@@ -117,7 +155,7 @@ int tiles_per_item(int kx, int group)
 }
 
 std::vector<BatchItem> make_items(const std::vector<int>& nx, const std::vector<int>& ny, const std::vector<int>& kx,
-	int order, int group)
+	const std::vector<int>& ky, int order, int group)
 {
 	const int n = static_cast<int>(nx.size());
 	std::vector<int> idx(n);
@@ -131,31 +169,39 @@ std::vector<BatchItem> make_items(const std::vector<int>& nx, const std::vector<
 	for (int i : idx) {
 		const int tx = tiles_of(nx[i]), ty = tiles_of(ny[i]), s = tiles_per_item(kx[i], group);
 		for (int r = 0; r < ty; ++r) {
-			for (int c = 0; c < tx; c += s) items.push_back(BatchItem{i, r * tx + c, std::min(s, tx - c), tx * ty});
+			for (int c = 0; c < tx; c += s) {
+				items.push_back(BatchItem{i, c * kBatchTile, r * kBatchTile, std::min(s, tx - c), tx * ty, kx[i], ky[i], 0});
+			}
 		}
 	}
 	return items;
 }
 
-// What a 64x64 tile of a kx x ky PSF costs: its taps plus kTileOverhead, what staging, hand-off
-// and the epilogue take beside them.
-constexpr float kTileOverhead = 60.0f;
-float tile_cost(int kx, int ky) { return static_cast<float>(kx) * static_cast<float>(ky) + kTileOverhead; }
+// What an item of a kx x ky PSF costs, in taps of a 64x64 tile: the taps of its 32x32 quadrants
+// that touch the image, and per tile kTileOverhead for staging, hand-off and epilogue (measured
+// with four CTAs per SM on 512x512 images: 2.6 SM-microseconds a tile plus 0.0187 per tap).
+constexpr float kTileOverhead = 140.0f;
+float item_cost(const BatchItem& item, int nx, int ny)
+{
+	const int cols = (std::min(nx, item.x0 + item.count * kBatchTile) - item.x0 + 31) / 32;
+	const int rows = (std::min(ny, item.y0 + kBatchTile) - item.y0 + 31) / 32;
+	return static_cast<float>(cols * rows) * 0.25f * static_cast<float>(item.kx * item.ky) +
+		kTileOverhead * static_cast<float>(item.count);
+}
 
 // The queues of make_items' list: one for the whole batch, or one per PSF width with the SMs
 // shared out in proportion to the widths' work (at least one SM each, largest remainders).
-BatchQueues make_queues(const std::vector<BatchItem>& items, const std::vector<int>& kx, const std::vector<int>& ky,
+BatchQueues make_queues(const std::vector<BatchItem>& items, const std::vector<int>& nx, const std::vector<int>& ny,
 	int order, int sms)
 {
 	BatchQueues q{};
 	q.sms = std::max(1, std::min(sms, kBatchSmTable));
 	double work[kBatchClasses] = {}, all = 0.0;
 	for (size_t i = 0; i < items.size(); ++i) {
-		const int image = items[i].image;
-		const bool next = i == 0 || (order == kOrderByWidth && kx[image] != kx[items[i - 1].image]);
+		const bool next = i == 0 || (order == kOrderByWidth && items[i].kx != items[i - 1].kx);
 		if (next) q.of[q.classes++] = BatchClass{static_cast<int>(i), 0, 0.0f};
 		++q.of[q.classes - 1].count;
-		const double c = static_cast<double>(items[i].count) * tile_cost(kx[image], ky[image]);
+		const double c = item_cost(items[i], nx[items[i].image], ny[items[i].image]);
 		work[q.classes - 1] += c;
 		all += c;
 	}
@@ -275,7 +321,9 @@ struct iane_gb_rl_batch {
 	std::vector<size_t> img_bytes;
 	std::vector<iane_gb::BatchItem> items; // one phase of the queue
 	iane_gb::BatchItem* d_items = nullptr;
-	size_t smem = 0;                       // dynamic shared memory of the launch
+	float* d_taps = nullptr;               // per image the PSF and the adjoint in padded rows
+	std::vector<size_t> tap_off;           // floats
+	size_t smem = 0;                       // shared memory of a tile and its taps
 	int blocks_per_sm = 1;                 // resident CTAs per SM the launch uses
 	int order = 0;                         // queue order (autotuned)
 	int group = 0;                         // item shapes by PSF width (autotuned, tiles_per_item)
@@ -285,6 +333,9 @@ struct iane_gb_rl_batch {
 	cudaStream_t capture = nullptr;
 	cudaGraphExec_t exec = nullptr;
 	std::string key;
+
+	// floats of one of image i's two padded tap arrays, a multiple of 4 (16-byte copies)
+	size_t taps_of(int i) const { return static_cast<size_t>(iane_gb::batch_tap_pitch(kx[i])) * ky[i]; }
 };
 
 namespace iane_gb {
@@ -314,11 +365,13 @@ int fill_images(const iane_gb_rl_batch* b, const DevView* obs, const DevView* es
 		st = encode_tensor_map_f32(&im.map_ratio, ratio, nx, ny, 1, pitch * 4, plane * 4, tile_pitch(kxi, 2),
 			kBatchTile + 2 * (kyi / 2));
 		if (st) return st;
-		rl_plan_fill_passes(b->plans[i], &im.pass_a, &im.pass_b, &im.epi_a, &im.epi_b, status);
+		TileArgs pass_a, pass_b;
+		rl_plan_fill_passes(b->plans[i], &pass_a, &pass_b, &im.epi_a, &im.epi_b, status);
 		im.epi_a.ratio = ratio;
 		im.epi_a.obs = obs[i].ptr;
 		for (int a = 0; a < 3; ++a) im.epi_a.os[a] = obs[i].stride[a];
 		im.epi_a.obs_u8 = obs[i].dtype == IANE_GB_U8;
+		im.epi_a.obs_rows = obs[i].dtype == IANE_GB_F32 && obs[i].stride[0] == 4;
 		im.epi_a.eps = eps;
 		im.epi_b.est = e_work;
 		im.epi_b.eps = eps;
@@ -327,13 +380,13 @@ int fill_images(const iane_gb_rl_batch* b, const DevView* obs, const DevView* es
 			for (int a = 0; a < 3; ++a) im.epi_b.outs[a] = est[i].stride[a];
 			im.epi_b.out_u8 = est[i].dtype == IANE_GB_U8;
 		}
-		im.kx = kxi;
-		im.tiles_x = tiles_of(nx);
-		im.tiles = tiles_of(nx) * tiles_of(ny);
+		im.taps[0] = b->d_taps + b->tap_off[i];
+		im.taps[1] = im.taps[0] + b->taps_of(i);
 		im.write_out_final = in_place || !est ? 0 : 1;
 		idesc[i].obs = obs[i];
 		if (est) idesc[i].est = est[i];
 		idesc[i].work = e_work;
+		idesc[i].parts = reinterpret_cast<double*>(ratio);
 		idesc[i].pitch = pitch;
 		idesc[i].in_place = in_place ? 1 : 0;
 	}
@@ -365,7 +418,6 @@ int build_graph(iane_gb_rl_batch* b, const DevView* obs, const DevView* est, int
 	int* status = device_status_ptr();
 	if (!status) return IANE_GB_CUDA_ERROR;
 
-	float* starts = reinterpret_cast<float*>(base + b->parts_off);
 	const BatchSync sync = sync_words(b, base);
 	cudaStream_t s0 = b->capture;
 	cudaGraph_t graph = nullptr;
@@ -380,16 +432,16 @@ int build_graph(iane_gb_rl_batch* b, const DevView* obs, const DevView* est, int
 		return abort_capture(cuda_fail(cudaGetLastError(), "batch: clear queue"));
 	}
 	if (init == IANE_GB_RL_INIT_MEAN) {
-		batch_mean_kernel<<<n, 256, 0, s0>>>(b->d_init, starts, eps);
+		batch_mean_kernel<<<dim3(n, kStartBlocks), 256, 0, s0>>>(b->d_init);
 	}
-	batch_init_kernel<<<dim3(n, 16), 256, 0, s0>>>(b->d_init, starts, eps, init);
+	batch_init_kernel<<<dim3(n, kStartBlocks), 256, 0, s0>>>(b->d_init, eps, init);
 	if (iterations > 0) {
-		const BatchQueues queues = make_queues(b->items, b->kx, b->ky, b->order, device_sm_count());
+		const BatchQueues queues = make_queues(b->items, b->nx, b->ny, b->order, device_sm_count());
 		st = launch_batch_persistent(b->d_images, b->d_items, queues, 2 * iterations, sync, status,
 			b->blocks_per_sm * device_sm_count(), b->smem, s0);
 		if (st) return abort_capture(st);
 	} else {
-		batch_init_kernel<<<dim3(n, 16), 256, 0, s0>>>(b->d_init, starts, eps, -1);
+		batch_init_kernel<<<dim3(n, kStartBlocks), 256, 0, s0>>>(b->d_init, eps, -1);
 	}
 	if (cudaGetLastError() != cudaSuccess) {
 		return abort_capture(cuda_fail(cudaGetLastError(), "batch: capture launches"));
@@ -483,11 +535,11 @@ int autotune(iane_gb_rl_batch* b, cudaStream_t stream)
 	float best = 0.0f;
 	// ms of a two-iteration run of the whole batch with one launch configuration
 	auto time_config = [&](int order, int group, int bps, float& ms) -> int {
-		const std::vector<BatchItem> items = make_items(b->nx, b->ny, b->kx, order, group);
+		const std::vector<BatchItem> items = make_items(b->nx, b->ny, b->kx, b->ky, order, group);
 		if (cudaMemcpy(d_items, items.data(), items.size() * sizeof(BatchItem), cudaMemcpyHostToDevice) != cudaSuccess) {
 			return cuda_fail(cudaGetLastError(), "autotune: upload items");
 		}
-		const BatchQueues queues = make_queues(items, b->kx, b->ky, order, sms);
+		const BatchQueues queues = make_queues(items, b->nx, b->ny, order, sms);
 		ms = 0.0f;
 		for (int rep = 0; rep < 3; ++rep) {
 			if (cudaMemsetAsync(sync.queue, 0, sync_bytes(n), stream) != cudaSuccess) {
@@ -548,6 +600,7 @@ int iane_gb_rl_batch_destroy(iane_gb_rl_batch* b)
 	if (!b) return IANE_GB_OK;
 	for (auto* p : b->plans) iane_gb_rl_destroy(p);
 	cudaFree(b->d_items);
+	cudaFree(b->d_taps);
 	cudaFree(b->d_images);
 	cudaFree(b->d_init);
 	if (b->exec) cudaGraphExecDestroy(b->exec);
@@ -602,7 +655,7 @@ int iane_gb_rl_batch_prepare(const iane_gb_view* psfs, int count, const int32_t*
 	b->scratch_bytes = off + kAlignB;
 	b->order = kOrderByWidth;
 	b->group = 0;
-	b->items = make_items(b->nx, b->ny, b->kx, b->order, b->group);
+	b->items = make_items(b->nx, b->ny, b->kx, b->ky, b->order, b->group);
 	b->blocks_per_sm = default_blocks_per_sm(b->items.size(), batch_blocks_per_sm(b->smem), device_sm_count());
 	if (cudaMalloc(&b->d_items, b->items.size() * sizeof(BatchItem)) != cudaSuccess ||
 	    cudaMalloc(&b->d_images, count * sizeof(BatchImage)) != cudaSuccess ||
@@ -610,10 +663,29 @@ int iane_gb_rl_batch_prepare(const iane_gb_view* psfs, int count, const int32_t*
 	    cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking) != cudaSuccess) {
 		return cleanup(cuda_fail(cudaGetLastError(), "rl_batch_prepare: allocate descriptors"));
 	}
+	size_t taps = 0;
+	for (int i = 0; i < count; ++i) {
+		b->tap_off.push_back(taps);
+		taps += 2 * b->taps_of(i);
+	}
+	if (cudaMalloc(&b->d_taps, taps * sizeof(float)) != cudaSuccess) {
+		return cleanup(cuda_fail(cudaGetLastError(), "rl_batch_prepare: allocate taps"));
+	}
+	for (int i = 0; i < count; ++i) {
+		TileArgs pa, pb;
+		EpiRatio ea;
+		EpiUpdate eb;
+		rl_plan_fill_passes(b->plans[i], &pa, &pb, &ea, &eb, nullptr);
+		batch_taps_kernel<<<1, 256, 0, static_cast<cudaStream_t>(stream)>>>(reinterpret_cast<const float*>(pa.kernel),
+			reinterpret_cast<const float*>(pb.kernel), b->kx[i], b->ky[i], batch_tap_pitch(b->kx[i]), b->d_taps + b->tap_off[i]);
+	}
+	if (cudaStreamSynchronize(static_cast<cudaStream_t>(stream)) != cudaSuccess) {
+		return cleanup(cuda_fail(cudaGetLastError(), "rl_batch_prepare: taps"));
+	}
 	if (flags & IANE_GB_BATCH_AUTOTUNE) {
 		const int st = autotune(b, static_cast<cudaStream_t>(stream));
 		if (st) return cleanup(st);
-		b->items = make_items(b->nx, b->ny, b->kx, b->order, b->group);
+		b->items = make_items(b->nx, b->ny, b->kx, b->ky, b->order, b->group);
 	}
 	if (cudaMemcpy(b->d_items, b->items.data(), b->items.size() * sizeof(BatchItem), cudaMemcpyHostToDevice) !=
 	    cudaSuccess) {
@@ -653,7 +725,7 @@ int iane_gb_rl_batch_configure(iane_gb_rl_batch* b, int blocks_per_sm, int order
 	    grouping < 0 || grouping >= kGroups) {
 		return fail(IANE_GB_INVALID_ARGUMENT, "rl_batch_configure: configuration out of range");
 	}
-	std::vector<BatchItem> items = make_items(b->nx, b->ny, b->kx, order, grouping);
+	std::vector<BatchItem> items = make_items(b->nx, b->ny, b->kx, b->ky, order, grouping);
 	// a run still in flight may read the queue: wait for the device before replacing it (a
 	// grouping never makes more items than one tile per item, for which d_items was sized)
 	IANE_GB_CUDA(cudaDeviceSynchronize(), "rl_batch_configure: wait for running work");

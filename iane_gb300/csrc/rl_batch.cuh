@@ -9,7 +9,8 @@
 // (BatchClass): the CTAs of an SM then stay on one width's code until its queue is empty. RL's only dependency is per image: a phase of an image reads
 // (with a halo) what the image's previous phase wrote and overwrites what it read, so an item
 // of phase p waits until all tiles of its image's phase p - 1 are done -- a per-image
-// completion counter that reaches p * tiles -- instead of a grid-wide drain between passes.
+// completion counter that reaches p * 4 * tiles, counted by warps -- instead of a grid-wide
+// drain between passes.
 // Images of the next phase start as soon as their own previous pass is complete.
 //
 // Progress: an item waits only for items earlier in the queue, which were handed to CTAs that
@@ -30,27 +31,26 @@ namespace iane_gb {
 // Tile edge of every work item (64 x 64 outputs; the body is 2 x 2 warps of 32 x 32).
 constexpr int kBatchTile = 64;
 
-// Device-side description of one image of the batch (64-byte aligned for the maps).
-struct alignas(64) BatchImage {
+// Device-side description of one image of the batch (128-byte aligned for the maps).
+struct alignas(128) BatchImage {
 	CUtensorMap map_est;   // TMA map of the work estimate (pass A source)
 	CUtensorMap map_ratio; // TMA map of the ratio image (pass B source)
-	TileArgs pass_a;       // kernel = PSF
-	TileArgs pass_b;       // kernel = adjoint
 	EpiRatio epi_a;
 	EpiUpdate epi_b;       // write_out is set only in the last iteration (write_out_final)
-	int kx;
-	int tiles_x;
-	int tiles;             // 64x64 tiles of this image (completions per phase)
+	const float* taps[2];  // PSF and adjoint, rows padded to a multiple of four taps (16-byte aligned)
 	int write_out_final;
 };
+static_assert(sizeof(BatchImage) % 16 == 0, "copied into shared memory in bulk");
 
-// `count` consecutive 64x64 tiles of one tile row of an image, from tile index `tile`: the
+// `count` consecutive 64x64 tiles of one tile row of an image: the
 // item's shape is (64 count) x 64 (count is 1, 2 or 4, chosen per PSF size by the autotuner).
-struct BatchItem {
+struct alignas(16) BatchItem {
 	int image;
-	int tile;
+	int x0, y0; // origin of the first tile
 	int count;
-	int image_tiles; // the image's 64x64 tiles (its completions per phase), read at hand-off
+	int image_tiles; // the image's 64x64 tiles (its completions per phase)
+	int kx, ky;
+	int reserved;
 };
 
 // Queues of one launch: at most one per PSF width (odd, 1 .. 31).
@@ -81,16 +81,19 @@ struct BatchSync {
 	unsigned int* done;
 };
 
-// The persistent launch (rl_batch_kernel.cu): `grid` CTAs of 128 threads, `smem` bytes of
-// dynamic shared memory (batch_tile_smem over the batch).
+// The persistent launch (rl_batch_kernel.cu): `grid` CTAs of 128 threads, `stage` bytes of shared
+// memory for a tile and its taps (batch_tile_smem over the batch).
 int launch_batch_persistent(const BatchImage* images, const BatchItem* items, const BatchQueues& queues, int phases,
-	BatchSync sync, int* status, int grid, size_t smem, cudaStream_t stream);
+	BatchSync sync, int* status, int grid, size_t stage, cudaStream_t stream);
 
-// Dynamic shared memory a tile of PSF width kx, height ky needs.
+// Shared memory that a tile of PSF width kx, height ky and its taps take.
 size_t batch_tile_smem(int kx, int ky);
 
-// Resident CTAs per SM of the persistent kernel with `smem` bytes of dynamic shared memory.
-int batch_blocks_per_sm(size_t smem);
+// Resident CTAs per SM of the persistent kernel with `stage` bytes for a tile and its taps.
+int batch_blocks_per_sm(size_t stage);
+
+// Floats of one padded tap row of a PSF kx wide.
+__host__ __device__ inline int batch_tap_pitch(int kx) { return (kx + 3) & ~3; }
 
 // Fill the plan-dependent fields of one image's pass arguments and epilogues (rl.cu); the
 // caller sets the buffer pointers, views and epsilon.

@@ -1,5 +1,5 @@
 // The persistent kernel of the batched Richardson-Lucy run (rl_batch.cuh): one launch takes
-// every (phase, image, tile) item of the run from a device queue, waits for the item's image
+// every (phase, image, tile) item of the run from the device queues, waits for the item's image
 // to finish its previous phase, runs the fused tiled convolution body of the item's pass and
 // PSF width, and counts the tile as done for its image.
 #include "rl_batch.cuh"
@@ -7,18 +7,36 @@
 namespace iane_gb {
 namespace {
 
-// Bytes after the tiles and taps: the two tile mbarriers and the item index.
-constexpr size_t kBatchTail = 32;
+// Shared memory: the halo tile and taps (`stage` bytes), then this.
+struct BatchShared {
+	BatchImage image[2]; // the descriptor of the tile in work and of the next one
+	int4 tile[2];        // phase (-1: the run is over), image, x0, y0
+	int2 taps[2];        // kx, ky
+	uint64_t full;       // tile, taps and descriptor have landed
+	// thread 0's own: the item in hand and which of its tiles comes next
+	BatchItem item;
+	int phase;           // of that item; -1: nothing is left
+	int next;
+	int cls;             // the queue it takes items from
+	unsigned int issued; // tiles handed on, the -1 included
+};
 
-// The sums of one item's tile for its PSF width (the epilogue is applied by the caller).
-__device__ __forceinline__ void item_sums(const BatchImage& im, bool pass_b, int x0, int y0, uint32_t& phases,
-	uint64_t* bars, float (&acc)[kRY][kRX], bool taps_resident)
+// The sums of one tile for its PSF width (the epilogue is applied by the caller): the body of
+// conv_tile_sums for a single kernel plane.
+template<int K>
+__device__ __forceinline__ void tile_sums(const float* tile, const float* taps, int ky, int t, float (&acc)[kRY][kRX])
 {
-	const CUtensorMap* map = pass_b ? &im.map_ratio : &im.map_est;
-	const TileArgs& a = pass_b ? im.pass_b : im.pass_a;
+	constexpr int P = TileWidth<K, 2>::P;
+	const int lane = t & 31, warp = t >> 5;
+	const int tx = (warp & 1) * 4 + (lane & 3), ty = (warp >> 1) * 8 + (lane >> 2);
+	plane_sums<K, P, kRX, kRY>(acc, tile + kRY * ty * P + kRX * tx, taps, ky / 2, ky);
+}
+
+__device__ __forceinline__ void item_sums(const float* tile, int kx, int ky, int t, float (&acc)[kRY][kRX])
+{
 #define IANE_GB_BATCH_KX(K) \
-	case K: conv_tile_sums<K, 2, 2, kTileTma, true>(map, a, x0, y0, 0, phases, bars, acc, taps_resident); break;
-	switch (im.kx) {
+	case K: tile_sums<K>(tile, tile + ((TileWidth<K, 2>::P * (kBatchTile + (ky & ~1)) + 31) & ~31), ky, t, acc); break;
+	switch (kx) {
 	IANE_GB_BATCH_KX(1) IANE_GB_BATCH_KX(3) IANE_GB_BATCH_KX(5) IANE_GB_BATCH_KX(7)
 	IANE_GB_BATCH_KX(9) IANE_GB_BATCH_KX(11) IANE_GB_BATCH_KX(13) IANE_GB_BATCH_KX(15)
 	IANE_GB_BATCH_KX(17) IANE_GB_BATCH_KX(19) IANE_GB_BATCH_KX(21) IANE_GB_BATCH_KX(23)
@@ -53,95 +71,169 @@ __device__ __forceinline__ int fullest_queue(const BatchQueues& q, const unsigne
 	return best;
 }
 
-// total = dynamic shared memory of the launch: the largest tile and taps + kBatchTail.
-//
-// What bounds it: the FP32 pipe for wide PSFs, latency for narrow ones. Sixteen widths of the
-// tile body are 419 KB of code, and with one queue for the whole batch the four CTAs of an SM
-// run different widths most of the time and stall on instruction fetch. With a queue per width
-// an SM's CTAs all start on the width that its id gives it (SMs are shared out by estimated
-// work, neighbours together, as they share instruction caches) and change only when that
-// width's queue is empty. 256 images of 64..1024 pixels a side, PSFs 3..31, 30 iterations: 62.4 ms
-// with one queue, largest images first, 37.7 ms with a queue per width.
-__global__ void __launch_bounds__(128) batch_persistent_kernel(const BatchImage* __restrict__ images,
-	const BatchItem* __restrict__ items, const __grid_constant__ BatchQueues queues, int phases, BatchSync sync,
-	int* status, unsigned int total)
+// tile_pitch(kx, 2) on the device.
+__device__ __forceinline__ int batch_pitch(int kx)
 {
-	extern __shared__ __align__(128) unsigned char smem_raw[];
-	uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + total - kBatchTail);
-	int2* shared_item = reinterpret_cast<int2*>(smem_raw + total - kBatchTail + 16);
-	int cls = 0; // thread 0's queue
-	if (threadIdx.x == 0) {
-		mbar_init(&bars[0], 1);
-		mbar_init(&bars[1], 1);
-		fence_barrier_init();
-		cls = queues.start[sm_id() % static_cast<unsigned int>(queues.sms)];
+	const int rx = kx / 2, rxa = (rx + 3) & ~3;
+	const int w = 64 - kRX + ((rxa - rx + kRX + kx - 1 + 3) & ~3);
+	return (w & 7) == 0 ? w + 4 : w;
+}
+
+struct FeedArgs {
+	const BatchImage* images;
+	const BatchItem* items;
+	int phases;
+	BatchSync sync;
+	int* status;
+	unsigned char* buffer;
+	BatchShared* sh;
+};
+
+// Thread 0: take the next tile in hand (the item's next one, or a new item's first).
+__device__ __forceinline__ void take_tile(const FeedArgs& a, const BatchQueues& queues)
+{
+	BatchShared& sh = *a.sh;
+	if (sh.phase >= 0 && sh.next + 1 < sh.item.count) {
+		++sh.next;
+		return;
 	}
-	uint32_t tile_phases = 0;
-	for (;;) {
-		__syncthreads(); // the previous item is finished everywhere; barriers initialised
-		if (threadIdx.x == 0) {
-			// (phase, item) of the next work item; phase -1: nothing left, or the run was aborted
-			int2 next = make_int2(-1, 0);
-			while (cls >= 0 && !load_volatile(sync.abort)) {
-				const BatchClass& q = queues.of[cls];
-				const unsigned int count = static_cast<unsigned int>(q.count);
-				const unsigned int k = atomicAdd(sync.queue + cls, 1u);
-				if (k < count * static_cast<unsigned int>(phases)) {
-					const unsigned int phase = k / count;
-					next = make_int2(static_cast<int>(phase), q.first + static_cast<int>(k - phase * count));
-					break;
-				}
-				cls = fullest_queue(queues, sync.queue, phases);
-			}
-			if (next.x >= 0) {
-				const BatchItem w = items[next.y];
-				// the item's tensor map into the descriptor cache while the wait and the taps proceed
-				const CUtensorMap* map = (next.x & 1) ? &images[w.image].map_ratio : &images[w.image].map_est;
-				asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
-				if (next.x > 0) {
-					// the image's previous phase complete (bounded: a wait that gives up aborts the run)
-					if (!wait_counter(&sync.done[w.image], static_cast<unsigned int>(next.x) * w.image_tiles, sync.abort,
-						status)) {
-						next.x = -1;
-					}
-					fence_proxy_async_global(); // the image's previous phase, written by generic stores, before TMA
-				}
-			}
-			*shared_item = next;
-		}
-		__syncthreads();
-		const int phase = shared_item->x;
-		if (phase < 0) {
+	int phase = -1, cls = sh.cls;
+	while (cls >= 0 && !load_volatile(a.sync.abort)) {
+		const BatchClass& q = queues.of[cls];
+		const unsigned int count = static_cast<unsigned int>(q.count);
+		const unsigned int k = atomicAdd(a.sync.queue + cls, 1u);
+		if (k < count * static_cast<unsigned int>(a.phases)) {
+			phase = static_cast<int>(k / count);
+			sh.item = a.items[q.first + static_cast<int>(k - static_cast<unsigned int>(phase) * count)];
+			sh.next = 0;
+			// the item's tensor map into the descriptor cache
+			const BatchImage* im = a.images + sh.item.image;
+			const CUtensorMap* map = (phase & 1) ? &im->map_ratio : &im->map_est;
+			asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 			break;
 		}
-		const BatchItem w = items[shared_item->y];
-		const BatchImage& im = images[w.image];
-		const int y0 = (w.tile / im.tiles_x) * kBatchTile;
-		// the item's tiles, left to right along one tile row; the PSF taps stay in shared memory
-		// from the first tile to the last
-		for (int c = 0; c < w.count; ++c) {
-			const int x0 = (w.tile % im.tiles_x + c) * kBatchTile;
-			float acc[kRY][kRX];
-			int xo = 0, yo = 0;
-			tile_origin<2>(x0, y0, xo, yo);
-			item_sums(im, phase & 1, x0, y0, tile_phases, bars, acc, c > 0);
-			if (phase & 1) {
-				EpiUpdate epi = im.epi_b; // read only after the sums: not live during them
-				epi.want_stats = 0;
-				epi.write_out = phase == phases - 1 && im.write_out_final;
+		cls = fullest_queue(queues, a.sync.queue, a.phases);
+	}
+	sh.phase = phase;
+	sh.cls = cls;
+}
+
+// Completions of the image's previous phases that the tile in hand needs (four warps a tile).
+__device__ __forceinline__ unsigned int tile_need(const BatchShared& sh)
+{
+	return static_cast<unsigned int>(sh.phase) * 4u * static_cast<unsigned int>(sh.item.image_tiles);
+}
+
+// Thread 0, the buffers being free and the image's previous phase complete: hand on the tile.
+__device__ __forceinline__ void issue_tile(const FeedArgs& a)
+{
+	BatchShared& sh = *a.sh;
+	const int slot = static_cast<int>(sh.issued++ & 1u);
+	const int x0 = sh.item.x0 + sh.next * kBatchTile, y0 = sh.item.y0;
+	sh.tile[slot] = make_int4(sh.phase, sh.item.image, x0, y0);
+	if (sh.phase < 0) {
+		mbar_arrive(&sh.full);
+		return;
+	}
+	const int kx = sh.item.kx, ky = sh.item.ky;
+	sh.taps[slot] = make_int2(kx, ky);
+	const BatchImage* im = a.images + sh.item.image;
+	const int pass_b = sh.phase & 1;
+	const uint32_t plane = static_cast<uint32_t>(batch_pitch(kx)) * static_cast<uint32_t>(kBatchTile + 2 * (ky / 2));
+	const uint32_t tap_bytes = static_cast<uint32_t>(batch_tap_pitch(kx) * ky * 4);
+	fence_proxy_async_global(); // the image's previous phase, written by generic stores, before TMA
+	// order earlier generic-proxy reads of the buffers before the async-proxy writes
+	asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+	mbar_arrive_expect_tx(&sh.full, plane * 4 + tap_bytes + static_cast<uint32_t>(sizeof(BatchImage)));
+	tma_load_3d(a.buffer, pass_b ? &im->map_ratio : &im->map_est, x0 - ((kx / 2 + 3) & ~3), y0 - ky / 2, 0, &sh.full);
+	bulk_copy_shared(a.buffer + ((plane + 31) & ~31u) * 4, im->taps[pass_b], tap_bytes, &sh.full);
+	bulk_copy_shared(&sh.image[slot], im, static_cast<uint32_t>(sizeof(BatchImage)), &sh.full);
+}
+
+// What bounds it: the FP32 pipe for wide PSFs, latency for narrow ones.
+//
+// Sixteen widths of the tile body are 419 KB of code, and with one queue for the whole batch the
+// four CTAs of an SM run different widths most of the time and stall on instruction fetch. With
+// a queue per width an SM's CTAs all start on the width that its id gives it (SMs are shared out
+// by estimated work, neighbours together, as they share instruction caches) and change only when
+// that width's queue is empty. 256 images of 64..1024 pixels a side, PSFs 3..31, 30 iterations:
+// 62.4 ms with one queue, largest images first, 37.7 ms with a queue per width, 33.1 ms with the
+// hand-off below (and the start values, 2 ms of it, from 32 blocks per image instead of one).
+//
+// The steps of the hand-off are spread over the tile before: its queue and item reads run while
+// that tile is still landing, its loads (tile, taps, descriptor, all asynchronous) start as soon
+// as the sums have read the buffers and land during the epilogue. A tile in hand never waits for
+// its image before the tile in work is counted done, so the earliest unfinished tile can always
+// proceed. Each warp counts itself done: no barrier follows the epilogue.
+__global__ void __launch_bounds__(128, 4) batch_persistent_kernel(const BatchImage* __restrict__ images,
+	const BatchItem* __restrict__ items, const __grid_constant__ BatchQueues queues, int phases, BatchSync sync,
+	int* status, unsigned int stage)
+{
+	extern __shared__ __align__(128) unsigned char smem_raw[];
+	BatchShared* sh = reinterpret_cast<BatchShared*>(smem_raw + stage);
+	const FeedArgs feed{images, items, phases, sync, status, smem_raw, sh};
+	const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+	if (t == 0) {
+		mbar_init(&sh->full, 1);
+		fence_barrier_init();
+		sh->phase = -1;
+		sh->issued = 0;
+		sh->cls = queues.start[sm_id() % static_cast<unsigned int>(queues.sms)];
+		take_tile(feed, queues);
+		if (sh->phase > 0 && !wait_counter(sync.done + sh->item.image, tile_need(*sh), sync.abort, status)) sh->phase = -1;
+	}
+	__syncthreads();
+	if (t == 0) issue_tile(feed);
+	const float* tile = reinterpret_cast<const float*>(smem_raw);
+	for (unsigned int n = 0;; ++n) {
+		if (t == 0) take_tile(feed, queues); // the tile after this one
+		if (!mbar_wait_bounded(&sh->full, n & 1)) {
+			report_device_status(status, IANE_GB_DEVICE_TIMEOUT);
+			atomicExch(sync.abort, 1);
+			return;
+		}
+		const int slot = n & 1;
+		const int4 m = sh->tile[slot];
+		const int phase = m.x;
+		if (phase < 0) return;
+		const int2 k = sh->taps[slot];
+		const BatchImage& im = sh->image[slot];
+		float acc[kRY][kRX];
 #pragma unroll
-				for (int j = 0; j < kRY; ++j) epi.row(xo, yo + j, 0, acc[j]);
-			} else {
-				const EpiRatio epi = im.epi_a;
+		for (int j = 0; j < kRY; ++j)
 #pragma unroll
-				for (int j = 0; j < kRY; ++j) epi.row(xo, yo + j, 0, acc[j]);
-			}
+			for (int i = 0; i < kRX; ++i) acc[j][i] = 0.0f;
+		const int wx = m.z + 32 * (warp & 1), wy = m.w + 32 * (warp >> 1);
+		// a warp whose 32 x 32 outputs all lie outside the image has nothing to sum or store
+		if (wx < im.epi_a.nx && wy < im.epi_a.ny) item_sums(tile, k.x, k.y, t, acc);
+		__syncthreads(); // tile and taps have been read
+		bool waiting = false;
+		if (t == 0) {
+			waiting = sh->phase > 0 && load_acquire(sync.done + sh->item.image) < tile_need(*sh);
+			if (!waiting) issue_tile(feed);
+		}
+		const int xo = wx + kRX * (lane & 3), yo = wy + kRY * (lane >> 2);
+		if (phase & 1) {
+			EpiUpdate epi = im.epi_b;
+			epi.want_stats = 0;
+			epi.write_out = phase == phases - 1 && im.write_out_final;
+#pragma unroll
+			for (int j = 0; j < kRY; ++j) epi.row(xo, yo + j, 0, acc[j]);
+		} else {
+			const EpiRatio epi = im.epi_a;
+#pragma unroll
+			for (int j = 0; j < kRY; ++j) epi.row(xo, yo + j, 0, acc[j]);
 		}
 		fence_proxy_async_global(); // this thread's epilogue stores, before other tiles' TMA reads
-		__syncthreads();
-		if (threadIdx.x == 0) {
+		__syncwarp();
+		if (lane == 0) {
 			__threadfence();
-			atomicAdd(&sync.done[w.image], static_cast<unsigned int>(w.count));
+			atomicAdd(&sync.done[m.y], 1u);
+		}
+		if (waiting) {
+			// bounded: a wait that gives up aborts the run
+			if (!wait_counter(sync.done + sh->item.image, tile_need(*sh), sync.abort, status)) sh->phase = -1;
+			issue_tile(feed);
 		}
 	}
 }
@@ -152,13 +244,13 @@ size_t batch_tile_smem(int kx, int ky)
 {
 	const int H = kBatchTile + 2 * (ky / 2);
 	const size_t plane = (static_cast<size_t>(tile_pitch(kx, 2)) * H * 4 + 127) & ~size_t(127);
-	const size_t taps = (static_cast<size_t>(ky) * ((kx + 3) & ~3) * 4 + 127) & ~size_t(127);
-	return plane + taps + 16; // 2-D images: one tile buffer and one tap buffer
+	const size_t taps = (static_cast<size_t>(ky) * batch_tap_pitch(kx) * 4 + 127) & ~size_t(127);
+	return plane + taps; // 2-D images: one tile buffer and one tap buffer
 }
 
-int batch_blocks_per_sm(size_t smem)
+int batch_blocks_per_sm(size_t stage)
 {
-	const size_t total = smem + kBatchTail;
+	const size_t total = stage + sizeof(BatchShared);
 	int per_sm = 0;
 	if (cudaFuncSetAttribute(batch_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	        static_cast<int>(total)) != cudaSuccess ||
@@ -170,16 +262,16 @@ int batch_blocks_per_sm(size_t smem)
 }
 
 int launch_batch_persistent(const BatchImage* images, const BatchItem* items, const BatchQueues& queues, int phases,
-	BatchSync sync, int* status, int grid, size_t smem, cudaStream_t stream)
+	BatchSync sync, int* status, int grid, size_t stage, cudaStream_t stream)
 {
 	if (queues.classes <= 0 || phases <= 0) {
 		return IANE_GB_OK;
 	}
-	const size_t total = smem + kBatchTail;
+	const size_t total = stage + sizeof(BatchShared);
 	IANE_GB_CUDA(cudaFuncSetAttribute(batch_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
 		static_cast<int>(total)), "batch: set shared memory size");
 	batch_persistent_kernel<<<grid, 128, total, stream>>>(images, items, queues, phases, sync, status,
-		static_cast<unsigned int>(total));
+		static_cast<unsigned int>(stage));
 	IANE_GB_CUDA(cudaGetLastError(), "batch: launch");
 	return IANE_GB_OK;
 }

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(128, 2) tc_conv_kernel(const __grid_constant__
 			for (int c = 0; c < kTcChunks; ++c) {
 				tma_load_3d(st + c * chunk_bytes, &map, x0 - kTcXA + 8 * c, y0 - ry, z + rz - qz, &full[s]);
 			}
-			tc::bulk_load(st + tile_bytes, a.tmat + static_cast<size_t>(qz) * ky * (kTcTmatBytes / 2), tmat_bytes, &full[s]);
+			bulk_copy_shared(st + tile_bytes, a.tmat + static_cast<size_t>(qz) * ky * (kTcTmatBytes / 2), tmat_bytes, &full[s]);
 		};
 		bool ok = true;
 		for (int p = 0; p < kTcStages && p < np; ++p) load(p);

@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kTczThreads) tcz_conv_kernel(const __grid_cons
 		mbar_arrive_expect_tx(tmat_bar, tmat_bytes);
 		const uint32_t row_bytes = tmat_bytes / ky;
 		for (int b = 0; b < ky; ++b) {
-			tc::bulk_load(tmat_s + b * row_bytes, reinterpret_cast<const unsigned char*>(a.tmat) + b * row_bytes, row_bytes,
+			bulk_copy_shared(tmat_s + b * row_bytes, reinterpret_cast<const unsigned char*>(a.tmat) + b * row_bytes, row_bytes,
 				tmat_bar);
 		}
 		auto load = [&](int p) {

@@ -95,13 +95,5 @@ __device__ __forceinline__ void ld_32x32b_x16(uint32_t taddr, float (&v)[16])
 	for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// 1-D bulk copy global -> shared completing on `bar` (16-byte aligned, size multiple of 16).
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar)
-{
-	asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-		::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar))
-		: "memory");
-}
-
 }  // namespace tc
 }  // namespace iane_gb

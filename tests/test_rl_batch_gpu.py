@@ -171,3 +171,29 @@ def test_every_item_shape_matches_the_single_image_path(cuda, grouping):
     with pytest.raises(iane_gb300.IaneError):
         batch.configure(1, 0, 4)
     batch.close()
+
+
+@pytest.mark.parametrize("shapes,ks", [
+    ([(300, 517)], [7]),                                            # one queue, items of one image
+    ([(33 + 3 * i, 65 - 2 * i) for i in range(16)], range(1, 32, 2)),  # sixteen queues, an item or two each
+    ([(1, 1), (65, 1), (1, 129), (64, 64), (128, 4)], [31, 1, 31, 3, 5]),  # single tiles, single pixels
+], ids=["one-queue", "all-widths", "tiny"])
+@pytest.mark.parametrize("mode", ["mean", "observed"])
+def test_queues_of_a_run_match_the_single_image_path(cuda, shapes, ks, mode):
+    # a queue per PSF width, tall PSFs among them; observed rows that are a crop of a wider frame
+    rng = np.random.default_rng(5)
+    obs = [rng.poisson(rng.random((ny, nx + 3)) * 100 + 5).astype(np.float32) for ny, nx in shapes]
+    psfs = [gaussian((k + 2 if k % 4 == 1 else k, k), (max(0.6, k / 5), max(0.6, k / 6))) for k in ks]
+    init = getattr(iane_gb300.RichardsonLucy, "INIT_" + mode.upper())
+    views = [to_gpu(o)[:, 1:1 + nx] for o, (ny, nx) in zip(obs, shapes)]
+    batch = iane_gb300.RichardsonLucyBatch([to_gpu(p) for p in psfs], shapes)
+    outs = [empty_like_np(s, np.float32) for s in shapes]
+    batch.run(views, outs, 5, 1e-6, init=init)
+    for v, p, g in zip(views, psfs, outs):
+        rl = iane_gb300.RichardsonLucy(to_gpu(p), tuple(v.shape))
+        e = empty_like_np(tuple(v.shape), np.float32)
+        rl.run(v, e, 5, 1e-6, init=init)
+        assert np.array_equal(to_host(g), to_host(e)), v.shape
+        rl.close()
+    iane_gb300.device_status()
+    batch.close()
