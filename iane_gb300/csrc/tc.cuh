@@ -95,5 +95,37 @@ __device__ __forceinline__ void ld_32x32b_x16(uint32_t taddr, float (&v)[16])
 	for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// Three such loads at once, with one wait.
+__device__ __forceinline__ void ld_32x32b_x16x3(uint32_t t0, uint32_t t1, uint32_t t2, float (&v0)[16], float (&v1)[16],
+	float (&v2)[16])
+{
+	uint32_t r[3][16];
+	const uint32_t t[3] = {t0, t1, t2};
+#pragma unroll
+	for (int k = 0; k < 3; ++k) {
+		asm volatile(
+			"tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+			: "=r"(r[k][0]), "=r"(r[k][1]), "=r"(r[k][2]), "=r"(r[k][3]), "=r"(r[k][4]), "=r"(r[k][5]), "=r"(r[k][6]),
+			  "=r"(r[k][7]), "=r"(r[k][8]), "=r"(r[k][9]), "=r"(r[k][10]), "=r"(r[k][11]), "=r"(r[k][12]), "=r"(r[k][13]),
+			  "=r"(r[k][14]), "=r"(r[k][15])
+			: "r"(t[k])
+			: "memory");
+	}
+	asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+	// no use of the registers moves above the wait
+#pragma unroll
+	for (int k = 0; k < 3; ++k) {
+		asm volatile("" : "+r"(r[k][0]), "+r"(r[k][1]), "+r"(r[k][2]), "+r"(r[k][3]), "+r"(r[k][4]), "+r"(r[k][5]), "+r"(r[k][6]),
+			"+r"(r[k][7]), "+r"(r[k][8]), "+r"(r[k][9]), "+r"(r[k][10]), "+r"(r[k][11]), "+r"(r[k][12]), "+r"(r[k][13]),
+			"+r"(r[k][14]), "+r"(r[k][15]));
+	}
+#pragma unroll
+	for (int i = 0; i < 16; ++i) {
+		v0[i] = __uint_as_float(r[0][i]);
+		v1[i] = __uint_as_float(r[1][i]);
+		v2[i] = __uint_as_float(r[2][i]);
+	}
+}
+
 }  // namespace tc
 }  // namespace iane_gb

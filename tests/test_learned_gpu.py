@@ -429,3 +429,55 @@ def test_learned_start_gains_over_the_flat_start(cuda):
     assert n_learn <= n_plain // 2, (n_learn, n_plain)
     rl32.close()
     rl16.close()
+
+
+@pytest.mark.parametrize("shape,c0,c1,co,masked", [
+    ((1, 1, 1), 8, 0, 8, False),       # one voxel, half a K step, half an N tile
+    ((3, 8, 14), 16, 0, 16, True),     # one tile exactly along x and y, an odd plane
+    ((2, 9, 15), 24, 0, 24, False),    # a second tile of one column and one row; ragged octets
+    ((5, 17, 29), 32, 16, 48, True),   # two inputs, two N tiles, the second ragged
+    ((4, 8, 28), 64, 0, 64, False),    # four K steps resident
+    ((2, 24, 30), 64, 32, 32, True),   # the most that stays resident
+    ((3, 10, 20), 128, 0, 32, False),  # too many weights to stay: the plain layout's SIMT kernel
+])
+def test_conv3_bf16_output_on_tensor_cores(cuda, shape, c0, c1, co, masked):
+    # BF16 operands' products are exact and the sums FP32, off by at most 1e-5 of the terms'
+    # magnitudes as in the FP32 tests; ReLU and rounding to BF16 are monotone, so a result lies
+    # between the roundings of the two ends of that interval
+    import torch
+
+    gen = torch.Generator().manual_seed(c0 * 100 + co + shape[2])
+    x0r, x0 = _act(gen, (c0,) + shape)
+    x1r, x1 = _act(gen, (max(c1, 8),) + shape)
+    mr, m = _act(gen, (co,) + shape)
+    wr, w = _bf16_tensor(gen, (co, c0 + c1, 27), 0.2)
+    b = torch.randn(co, generator=gen, dtype=torch.float32) * 0.1
+    bd = b.to(cuda)
+    y = to_c8(torch.full((co,) + shape, 7.0, dtype=torch.bfloat16, device=cuda))
+    _check(_lib().iane_gb_cnn_conv3(_p(x0), c0, _p(x1) if c1 else None, c1, *shape, _p(w), _p(bd), co, _p(y), None,
+                                    None, 1, _p(m) if masked else None, None))
+    torch.cuda.synchronize()
+    inp = torch.cat([x0r, x1r[:c1]], 0) if c1 else x0r
+    bias = b.double().view(-1, 1, 1, 1)
+    ref = conv3(inp, wr) + bias
+    off = 1e-5 * (conv3(inp.abs(), wr.abs()) + bias.abs())
+    got = from_c8(y.cpu(), co).double()
+    keep = (mr > 0).double() if masked else 1.0
+    lo, hi = (bf16_round(torch.relu(v)) * keep for v in (ref - off, ref + off))
+    assert bool(((got >= lo) & (got <= hi)).all())
+
+
+def test_conv3_tc_streams_weights_that_do_not_fit(cuda):
+    import torch
+
+    gen = torch.Generator().manual_seed(5)
+    shape, c, co = (5, 12, 33), 144, 40
+    xr, x = _act(gen, (c,) + shape)
+    wr, w = _bf16_tensor(gen, (co, c, 27), 0.1)
+    packed = torch.empty(int(_lib().iane_gb_cnn_tc_packed_bytes(co, c, 0)) // 2, dtype=torch.bfloat16, device=cuda)
+    _check(_lib().iane_gb_cnn_tc_pack(_p(w), co, c, 0, _p(packed), None))
+    y = torch.empty((co,) + shape, dtype=torch.float32, device=cuda)
+    _check(_lib().iane_gb_cnn_conv3_tc(_p(x), c, None, 0, *shape, _p(packed), None, co, None, _p(y), None, 0, None))
+    torch.cuda.synchronize()
+    ref, mag = conv3(xr, wr), conv3(xr.abs(), wr.abs())
+    assert float(((y.cpu().double() - ref).abs() / mag).max()) < 1e-5
