@@ -481,3 +481,37 @@ def test_conv3_tc_streams_weights_that_do_not_fit(cuda):
     torch.cuda.synchronize()
     ref, mag = conv3(xr, wr), conv3(xr.abs(), wr.abs())
     assert float(((y.cpu().double() - ref).abs() / mag).max()) < 1e-5
+
+
+@pytest.mark.parametrize("shape,c0,c1,co", [
+    ((1, 1, 1), 8, 0, 1),          # one voxel: every tap but the centre falls outside
+    ((3, 5, 17), 40, 0, 17),       # a second column of one voxel, a half pair of rows, ragged groups and tiles
+    ((2, 4, 65), 32, 8, 16),       # 80 voxels: five columns of 16
+    ((70, 2, 64), 16, 0, 64),      # planes in several runs
+    ((48, 48, 64), 16, 0, 16),     # accumulator sets taken in turn several times over
+])
+def test_conv3_weight_gradient_on_tensor_cores(cuda, shape, c0, c1, co):
+    # as test_conv3_weight_gradient: 1e-5 of the terms' magnitudes, and the rounding of the result
+    import torch
+
+    gen = torch.Generator().manual_seed(7 * c0 + co + shape[0])
+    x0r, x0 = _act(gen, (c0,) + shape)
+    x1r, x1 = _act(gen, (max(c1, 8),) + shape)
+    dyr, dy = _act(gen, (co,) + shape)
+    inp = torch.cat([x0r, x1r[:c1]], 0) if c1 else x0r
+    wants = []
+    for a, b in ((inp, dyr), (inp.abs(), dyr.abs())):
+        p = torch.nn.functional.pad(a, (1, 1, 1, 1, 1, 1))
+        d, h, w = shape
+        rows = [p[:, t // 9:t // 9 + d, t // 3 % 3:t // 3 % 3 + h, t % 3:t % 3 + w].reshape(c0 + c1, -1) for t in range(27)]
+        wants.append((torch.stack([b.reshape(co, -1) @ r.T for r in rows], 2), b.reshape(co, -1).sum(1)))
+    dw = torch.zeros((co, c0 + c1, 27), dtype=torch.float32, device=cuda)
+    db = torch.zeros(co, dtype=torch.float32, device=cuda)
+    need = _lib().iane_gb_cnn_wgrad_scratch_bytes(c0, c1, *shape, co)
+    scratch = torch.empty(int(need), dtype=torch.uint8, device=cuda)
+    _check(_lib().iane_gb_cnn_conv3_wgrad(_p(x0), c0, _p(x1) if c1 else None, c1, *shape, _p(dy), co, _p(dw), _p(db),
+                                          _p(scratch), scratch.numel(), None))
+    torch.cuda.synchronize()
+    for got, want, mag in zip((dw, db), *wants):
+        err = (got.cpu().double() - want).abs()
+        assert bool((err <= 1e-5 * mag + 2 ** -22 * want.abs() + 1e-30).all()), float((err - 1e-5 * mag).max())
