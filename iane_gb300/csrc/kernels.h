@@ -70,6 +70,11 @@ int launch_conv_separable_fast(const DevView& src, const DevView* taps, const De
 int launch_separable_rows(const DevView& src, const DevView* taps, const DevView& dst, int border,
 	cudaStream_t stream);
 
+// Box erosion / dilation of 2-D planes with radii up to 4, 8- and 16-bit integers and f32
+// (morphology_2d.cu); IANE_GB_UNSUPPORTED without an error when it does not apply.
+int launch_morph_planes(const DevView& src, const DevView& dst, const int* radius, bool dilate, int border,
+	cudaStream_t stream);
+
 // Fused separable FP32 convolution, any tap length (separable.cu).
 int launch_conv_separable(const DevView& src, const DevView* taps, const DevView& dst, int border,
 	cudaStream_t stream);

@@ -414,6 +414,8 @@ int launch_op(const DevView& s, const DevView& d, const int* r, const uint8_t* m
 		IANE_GB_CUDA(cudaGetLastError(), "morphology: launch");
 		return IANE_GB_OK;
 	}
+	const int planes = launch_morph_planes(s, d, r, DILATE, border, st);
+	if (planes != IANE_GB_UNSUPPORTED) return planes;
 	const size_t smem = box_xy_smem(r[0], r[1], sizeof(T));
 	if (smem > 200 * 1024) {
 		morph_direct_kernel<T, DILATE><<<g8, dim3(32, 8), 0, st>>>(s, d, r[0], r[1], r[2], nullptr, border);

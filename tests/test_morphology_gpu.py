@@ -177,3 +177,35 @@ def test_cube_footprint_with_a_plane_beyond_31_bit_offsets(cuda):
         iane_gb300.morphology(view, out, (1, 1, 1), op, "clamp")
         assert to_host(out).tobytes() == ref.tobytes(), op
     del buf
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.int8, np.uint16, np.int16, np.float32], ids=lambda d: np.dtype(d).name)
+@pytest.mark.parametrize("shape,radius", [
+    ((1, 1), (1, 1)), ((9, 7), (4, 4)),            # everything is border
+    ((8, 24), (1, 2)), ((17, 31), (2, 1)),         # one thread inside a row; an odd tail
+    ((33, 263), (3, 3)), ((40, 256), (0, 4)),      # several warps, a row's last element alone; whole groups
+    ((5, 19, 530), (0, 2, 1)),                     # a stack of planes
+    ((700, 2101), (4, 3)), ((640, 1024), (3, 4)),  # radii of 3 and 4 on larger images (integers; f32)
+])
+def test_planes_of_packed_rows(cuda, dtype, shape, radius):
+    # rows of every alignment: the packed image, and a crop whose rows start one element in
+    rng = np.random.default_rng(zlib.crc32(repr((np.dtype(dtype).name, shape, radius)).encode()))
+    wide = (*shape[:-1], shape[-1] + 2)
+    if dtype == np.float32:
+        big = rng.standard_normal(wide).astype(dtype)
+        for value in (np.nan, 0.0, -0.0, np.inf):
+            big[rng.random(wide) < 0.05] = value
+    else:
+        info = np.iinfo(dtype)
+        big = rng.integers(info.min, info.max, wide, dtype=dtype, endpoint=True)
+    for op in ("erode", "dilate"):
+        for border in ("clamp", "zero", "mirror"):
+            src = np.ascontiguousarray(big[..., 1:-1])
+            ref = np.zeros_like(src)
+            oracle.morphology(src, ref, radius, op, border)
+            assert run_gpu(src, radius, op, border).tobytes() == ref.tobytes(), (op, border)
+            g, out = to_gpu(big), to_gpu(np.zeros_like(big))
+            iane_gb300.morphology(g[..., 1:-1], out[..., 1:-1], radius, op, border)
+            got = to_host(out)
+            assert np.ascontiguousarray(got[..., 1:-1]).tobytes() == ref.tobytes(), (op, border, "crop")
+            assert not got[..., 0].any() and not got[..., -1].any()
