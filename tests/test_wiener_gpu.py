@@ -96,3 +96,24 @@ def test_wiener_errors(cuda):
     with pytest.raises(iane_gb300.IaneLengthError):
         w.run(obs, empty_like_np((32, 32), np.uint8), scratch=torch().empty(16, dtype=torch().uint8, device="cuda"))
     w.close()
+
+
+@pytest.mark.parametrize("shape", [(7, 5), (3, 1025), (2, 4099), (2, 3, 4096)], ids=str)
+@pytest.mark.parametrize("dtype", [np.uint8, np.float32], ids=lambda d: np.dtype(d).name)
+def test_aligned_and_unaligned_rows_give_the_same_bits(cuda, shape, dtype):
+    # packed images take word loads and stores where rows allow; crops that start one element into
+    # a wider frame take the element path: the transforms see the same values either way
+    rng = np.random.default_rng(sum(shape))
+    src = rng.integers(0, 256, shape).astype(dtype)
+    psf = np.full((1,) * (len(shape) - 1) + (3,), 1 / 3, np.float32)
+    plan = iane_gb300.Wiener(to_gpu(psf), shape, 0.01)
+    packed = empty_like_np(shape, dtype)
+    plan.run(to_gpu(src), packed)
+    wide = np.zeros((*shape[:-1], shape[-1] + 3), dtype)
+    wide[..., 1:-2] = src
+    out = to_gpu(np.zeros_like(wide))
+    plan.run(to_gpu(wide)[..., 1:-2], out[..., 1:-2])
+    got = to_host(out)
+    assert np.ascontiguousarray(got[..., 1:-2]).tobytes() == to_host(packed).tobytes()
+    assert not got[..., 0].any() and not got[..., -2:].any()
+    plan.close()
