@@ -37,12 +37,24 @@ __all__ = [
 ]
 
 
-def _stream_handle(stream) -> int:
-    import torch
+_raw_stream = None
 
-    if stream is None:
-        stream = torch.cuda.current_stream()
-    return int(stream.cuda_stream)
+
+def _stream_handle(stream) -> int:
+    """The CUDA handle of ``stream``, or of the current device's current stream."""
+    global _raw_stream
+    if stream is not None:
+        return int(stream.cuda_stream)
+    if _raw_stream is None:
+        import torch
+
+        torch.cuda.current_stream()  # initialises CUDA
+        # the handle without a Stream object around it, where this torch offers that (0.3 against
+        # 3 us of a call)
+        raw, device = (getattr(torch._C, n, None) for n in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
+        _raw_stream = ((lambda: raw(device())) if raw and device
+                       else (lambda: int(torch.cuda.current_stream().cuda_stream)))
+    return _raw_stream()
 
 
 def _border(border) -> int:
@@ -59,6 +71,19 @@ def _device_view(t) -> abi.View:
     return abi.torch_view(t)
 
 
+def _view_bytes(t) -> bytes:
+    """The same view as the bytes that a view argument takes too."""
+    if not t.is_cuda:
+        raise ValueError("iane_gb300 works on CUDA tensors; copy host data to the device first")
+    return abi.torch_view_bytes(t)
+
+
+_I32x3 = ctypes.c_int32 * 3
+
+
+_METHODS = {"direct": abi.ACC_FAST, "fft": abi.ACC_FAST | abi.CONV_FFT, "auto": abi.ACC_FAST | abi.CONV_AUTO}
+
+
 def convolve(src, kernel, dst, border="clamp", exact: bool = False, method: str = "direct", stream=None):
     """Convolution of ``src`` with ``kernel`` into ``dst`` (all CUDA tensors).
 
@@ -67,19 +92,19 @@ def convolve(src, kernel, dst, border="clamp", exact: bool = False, method: str 
     (int64 for integer image/kernel pairs). ``method="fft"`` uses the spectral path (FP64
     cuFFT transforms of the border-padded source; float types), ``method="auto"`` picks
     direct or spectral by a cost model. Asynchronous on ``stream``."""
-    if method not in ("direct", "fft", "auto"):
+    flags = _METHODS.get(method)
+    if flags is None:
         raise ValueError(f"unknown method {method!r}")
-    flags = abi.ACC_EXACT if exact else abi.ACC_FAST
-    flags |= {"direct": 0, "fft": abi.CONV_FFT, "auto": abi.CONV_AUTO}[method]
-    k, d = _device_view(kernel), _device_view(dst)
+    if exact:
+        flags |= abi.ACC_EXACT
+    k, d = _view_bytes(kernel), _view_bytes(dst)
     if isinstance(src, TextureView):
         tv = src._abi()
-        check(lib().iane_gb_convolve_texture(ctypes.byref(tv), ctypes.byref(k), ctypes.byref(d), _border(border),
-                                             flags, _stream_handle(stream)))
+        check(lib().iane_gb_convolve_texture(ctypes.byref(tv), k, d, _border(border), flags, _stream_handle(stream)))
         return dst
-    s = _device_view(src)
-    check(lib().iane_gb_convolve(ctypes.byref(s), ctypes.byref(k), ctypes.byref(d), _border(border), flags,
-                                 _stream_handle(stream)))
+    status = lib().iane_gb_convolve(_view_bytes(src), k, d, _border(border), flags, _stream_handle(stream))
+    if status:
+        check(status)
     return dst
 
 
@@ -109,12 +134,12 @@ def morphology(src, dst, radius, op: str = "erode", border="clamp", footprint=No
     when None) and may run in place (``src is dst``); erode and dilate need disjoint views."""
     if op not in abi.MORPHOLOGY_OPS:
         raise ValueError(f"unknown morphology op {op!r}")
-    s, d = _device_view(src), _device_view(dst)
+    s, d = _view_bytes(src), _view_bytes(dst)
     rank = len(src.shape)
     radius = tuple(int(r) for r in radius)
     if len(radius) != rank:
         raise ValueError("radius needs one entry per axis")
-    r = (ctypes.c_int32 * 3)(*([radius[rank - 1 - i] for i in range(rank)] + [0] * (3 - rank)))
+    r = _I32x3(*radius[::-1])
     mask = None
     if footprint is not None:
         if tuple(footprint.shape) != tuple(2 * v + 1 for v in radius) or not footprint.is_cuda:
@@ -123,17 +148,18 @@ def morphology(src, dst, radius, op: str = "erode", border="clamp", footprint=No
     code = abi.MORPHOLOGY_OPS[op]
     mp = None if mask is None else mask.data_ptr()
     if code in (abi.ERODE, abi.DILATE):
-        check(lib().iane_gb_morphology(ctypes.byref(s), ctypes.byref(d), r, mp, code, _border(border),
-                                       _stream_handle(stream)))
-        return dst
-    ext = (ctypes.c_int32 * 3)(*[s.extent[i] for i in range(3)])
-    need = int(lib().iane_gb_morphology_scratch_bytes(s.dtype, rank, ext))
-    if scratch is None:
-        import torch
+        status = lib().iane_gb_morphology(s, d, r, mp, code, _border(border), _stream_handle(stream))
+    else:
+        if scratch is None:
+            import torch
 
-        scratch = torch.empty(max(need, 1), dtype=torch.uint8, device=src.device)
-    check(lib().iane_gb_morphology_compound(ctypes.byref(s), ctypes.byref(d), r, mp, code, _border(border),
-                                            scratch.data_ptr(), scratch.numel(), _stream_handle(stream)))
+            ext = _I32x3(*tuple(src.shape)[::-1])
+            need = int(lib().iane_gb_morphology_scratch_bytes(abi.torch_view(src).dtype, rank, ext))
+            scratch = torch.empty(max(need, 1), dtype=torch.uint8, device=src.device)
+        status = lib().iane_gb_morphology_compound(s, d, r, mp, code, _border(border), scratch.data_ptr(),
+                                                   scratch.numel(), _stream_handle(stream))
+    if status:
+        check(status)
     return dst
 
 
@@ -159,8 +185,7 @@ class Wiener:
 
         if scratch is None:
             scratch = torch.empty(self.scratch_bytes, dtype=torch.uint8, device=observed.device)
-        s, d = _device_view(observed), _device_view(restored)
-        check(lib().iane_gb_wiener_run(self._plan, ctypes.byref(s), ctypes.byref(d), scratch.data_ptr(),
+        check(lib().iane_gb_wiener_run(self._plan, _view_bytes(observed), _view_bytes(restored), scratch.data_ptr(),
                                        scratch.numel(), _stream_handle(stream)))
         return restored
 
@@ -249,11 +274,14 @@ class TextureView:
 def convolve_separable(src, taps, dst, border="clamp", stream=None):
     """Convolution with the outer product of 1-D f32 ``taps`` (``taps[i]`` for IANE axis i,
     i.e. ``taps[0]`` runs along the last tensor dimension)."""
-    s, d = _device_view(src), _device_view(dst)
-    views = [_device_view(t) for t in taps]
-    arr = (ctypes.POINTER(abi.View) * max(1, len(views)))(*[ctypes.pointer(v) for v in views])
-    check(lib().iane_gb_convolve_separable(ctypes.byref(s), arr, ctypes.byref(d), _border(border),
-                                           _stream_handle(stream)))
+    s, d = _view_bytes(src), _view_bytes(dst)
+    views = [_view_bytes(t) for t in taps]
+    block = ctypes.create_string_buffer(b"".join(views))
+    first = ctypes.addressof(block)
+    arr = (ctypes.c_void_p * max(1, len(views)))(*[first + abi.VIEW_BYTES * i for i in range(len(views))])
+    status = lib().iane_gb_convolve_separable(s, arr, d, _border(border), _stream_handle(stream))
+    if status:
+        check(status)
     return dst
 
 
@@ -320,13 +348,13 @@ class RichardsonLucy:
             raise RuntimeError("plan destroyed")
         if scratch is None:
             scratch = torch.empty(self.scratch_bytes, dtype=torch.uint8, device=observed.device)
-        o, e = _device_view(observed), _device_view(estimate)
+        o, e = _view_bytes(observed), _view_bytes(estimate)
         stats_ptr = None
         if stats is not None:
             if stats.dtype != torch.float64 or not stats.is_cuda or stats.numel() < 2 * iterations:
                 raise ValueError("stats must be a CUDA float64 tensor with 2*iterations entries")
             stats_ptr = stats.data_ptr()
-        check(lib().iane_gb_rl_run(self._plan, ctypes.byref(o), ctypes.byref(e), int(iterations),
+        check(lib().iane_gb_rl_run(self._plan, o, e, int(iterations),
                                    ctypes.c_float(epsilon), int(init), scratch.data_ptr(), scratch.numel(),
                                    stats_ptr, _stream_handle(stream)))
         return estimate

@@ -49,6 +49,7 @@ def lib() -> ctypes.CDLL:
         raise RuntimeError(f"{LIB_PATH} is missing: build it with `python -m iane_gb300.build`")
     l = ctypes.CDLL(str(LIB_PATH))
     vp, cvp, i32p = ctypes.c_void_p, ctypes.c_void_p, ctypes.POINTER(ctypes.c_int32)
+    # view arguments take a View by reference or its bytes (abi.torch_view_bytes)
     l.iane_gb_abi_version.argtypes = []
     l.iane_gb_abi_version.restype = ctypes.c_int
     l.iane_gb_last_error.argtypes = [ctypes.c_char_p, ctypes.c_size_t]
@@ -59,9 +60,9 @@ def lib() -> ctypes.CDLL:
     l.iane_gb_wait_probe.restype = ctypes.c_int
     l.iane_gb_fp32_peak_probe.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_double), vp]
     l.iane_gb_fp32_peak_probe.restype = ctypes.c_int
-    l.iane_gb_convolve.argtypes = [_VIEW_P, _VIEW_P, _VIEW_P, ctypes.c_int, ctypes.c_uint, vp]
+    l.iane_gb_convolve.argtypes = [vp, vp, vp, ctypes.c_int, ctypes.c_uint, vp]
     l.iane_gb_convolve.restype = ctypes.c_int
-    l.iane_gb_convolve_separable.argtypes = [_VIEW_P, ctypes.POINTER(_VIEW_P), _VIEW_P, ctypes.c_int, vp]
+    l.iane_gb_convolve_separable.argtypes = [vp, vp, vp, ctypes.c_int, vp]
     l.iane_gb_convolve_separable.restype = ctypes.c_int
     l.iane_gb_rl_prepare.argtypes = [_VIEW_P, ctypes.c_int, i32p, vp, ctypes.POINTER(vp)]
     l.iane_gb_rl_prepare.restype = ctypes.c_int
@@ -69,7 +70,7 @@ def lib() -> ctypes.CDLL:
     l.iane_gb_rl_prepare_ex.restype = ctypes.c_int
     l.iane_gb_rl_scratch_bytes.argtypes = [cvp]
     l.iane_gb_rl_scratch_bytes.restype = ctypes.c_size_t
-    l.iane_gb_rl_run.argtypes = [vp, _VIEW_P, _VIEW_P, ctypes.c_int, ctypes.c_float, ctypes.c_int, vp,
+    l.iane_gb_rl_run.argtypes = [vp, vp, vp, ctypes.c_int, ctypes.c_float, ctypes.c_int, vp,
                                  ctypes.c_size_t, vp, vp]
     l.iane_gb_rl_run.restype = ctypes.c_int
     l.iane_gb_rl_host_scratch_bytes.argtypes = [cvp, ctypes.c_int]
@@ -119,18 +120,18 @@ def lib() -> ctypes.CDLL:
     l.iane_gb_texture_create.argtypes = [i, i, i32p, ctypes.POINTER(u64)]
     l.iane_gb_texture_upload.argtypes = [u64, _VIEW_P, vp]
     l.iane_gb_texture_destroy.argtypes = [u64]
-    l.iane_gb_convolve_texture.argtypes = [ctypes.POINTER(abi.TextureView), _VIEW_P, _VIEW_P, i, ctypes.c_uint, vp]
+    l.iane_gb_convolve_texture.argtypes = [ctypes.POINTER(abi.TextureView), vp, vp, i, ctypes.c_uint, vp]
     u8p = ctypes.c_void_p
-    l.iane_gb_morphology.argtypes = [_VIEW_P, _VIEW_P, i32p, u8p, i, i, vp]
+    l.iane_gb_morphology.argtypes = [vp, vp, i32p, u8p, i, i, vp]
     l.iane_gb_morphology.restype = ctypes.c_int
     l.iane_gb_morphology_scratch_bytes.argtypes = [i, i, i32p]
     l.iane_gb_morphology_scratch_bytes.restype = sz
-    l.iane_gb_morphology_compound.argtypes = [_VIEW_P, _VIEW_P, i32p, u8p, i, i, vp, sz, vp]
+    l.iane_gb_morphology_compound.argtypes = [vp, vp, i32p, u8p, i, i, vp, sz, vp]
     l.iane_gb_morphology_compound.restype = ctypes.c_int
     l.iane_gb_wiener_prepare.argtypes = [_VIEW_P, i, i32p, f, vp, ctypes.POINTER(vp)]
     l.iane_gb_wiener_scratch_bytes.argtypes = [cvp]
     l.iane_gb_wiener_scratch_bytes.restype = sz
-    l.iane_gb_wiener_run.argtypes = [vp, _VIEW_P, _VIEW_P, vp, sz, vp]
+    l.iane_gb_wiener_run.argtypes = [vp, vp, vp, vp, sz, vp]
     l.iane_gb_wiener_destroy.argtypes = [vp]
     for name in ("wiener_prepare", "wiener_run", "wiener_destroy"):
         getattr(l, "iane_gb_" + name).restype = ctypes.c_int

@@ -9,6 +9,7 @@ A C-ordered array of shape ``(nz, ny, nx)`` is therefore the IANE view with exte
 from __future__ import annotations
 
 import ctypes
+import struct
 
 ABI_VERSION = 2
 MAX_RANK = 3
@@ -120,3 +121,36 @@ def torch_view(t) -> View:
         raise TypeError(f"unsupported torch dtype {t.dtype}")
     size = t.element_size()
     return make_view(t.data_ptr(), code, tuple(t.shape), tuple(s * size for s in t.stride()))
+
+
+# The bytes of a View (the struct has no padding), for callers that only pass it on: packing them
+# takes a third of the time of filling a ctypes structure field by field.
+_VIEW_STRUCT = struct.Struct("=Qii3ii3q")
+assert _VIEW_STRUCT.size == ctypes.sizeof(View)
+VIEW_BYTES = _VIEW_STRUCT.size
+_torch_codes = {}  # torch dtype -> (code, element size)
+
+
+def torch_view_bytes(t) -> bytes:
+    """``bytes(torch_view(t))``."""
+    known = _torch_codes.get(t.dtype)
+    if known is None:
+        code = _TORCH_DTYPES.get(str(t.dtype))
+        if code is None:
+            raise TypeError(f"unsupported torch dtype {t.dtype}")
+        known = _torch_codes[t.dtype] = (code, t.element_size())
+    code, size = known
+    shape, stride = t.shape, t.stride()
+    try:
+        rank = len(shape)
+        if rank == 2:
+            return _VIEW_STRUCT.pack(t.data_ptr(), code, 2, shape[1], shape[0], 0, 0, stride[1] * size,
+                                     stride[0] * size, 0)
+        if rank == 3:
+            return _VIEW_STRUCT.pack(t.data_ptr(), code, 3, shape[2], shape[1], shape[0], 0, stride[2] * size,
+                                     stride[1] * size, stride[0] * size)
+        if rank == 1:
+            return _VIEW_STRUCT.pack(t.data_ptr(), code, 1, shape[0], 0, 0, 0, stride[0] * size, 0, 0)
+    except struct.error:
+        pass
+    return bytes(torch_view(t))

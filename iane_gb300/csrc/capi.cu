@@ -3,6 +3,7 @@
 #include "common.cuh"
 #include "kernels.h"
 
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -171,12 +172,15 @@ int encode_tensor_map_nd(CUtensorMap* map, int data_type, int rank, const void* 
 
 int device_sm_count()
 {
+	static std::atomic<int> cached[64] = {}; // by device
 	int device = 0;
 	int count = 0;
-	if (cudaGetDevice(&device) != cudaSuccess ||
-	    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || count <= 0) {
+	if (cudaGetDevice(&device) != cudaSuccess) return 148;
+	if (device >= 0 && device < 64 && (count = cached[device].load(std::memory_order_relaxed)) > 0) return count;
+	if (cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || count <= 0) {
 		return 148;
 	}
+	if (device >= 0 && device < 64) cached[device].store(count, std::memory_order_relaxed);
 	return count;
 }
 

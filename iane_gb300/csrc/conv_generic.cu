@@ -167,8 +167,10 @@ int launch_typed(const GenericArgs& args, cudaStream_t stream)
 	a.staged = coef_bytes + tile_bytes <= kLimit ? 1 : 0;
 	const size_t smem = coef_bytes + (a.staged ? tile_bytes : 0);
 	auto kernel = conv_generic_kernel<TS, TAcc>;
-	IANE_GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-		"convolve: set shared memory size");
+	if (smem > 48 * 1024) { // what a launch may use without asking
+		IANE_GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+			"convolve: set shared memory size");
+	}
 	const dim3 grid((a.src.ext[0] + kGX - 1) / kGX, (a.src.ext[1] + kGY - 1) / kGY, a.src.ext[2]);
 	kernel<<<grid, dim3(kGX, kGY), smem, stream>>>(a);
 	IANE_GB_CUDA(cudaGetLastError(), "convolve: launch generic kernel");

@@ -152,3 +152,17 @@ def test_wiener_argument_checks():
         abi.INVALID_ARGUMENT
     assert "PSF must fit inside the input image" in _lib.last_error()
     assert lib.iane_gb_wiener_run(None, None, None, None, 0, None) == abi.INVALID_ARGUMENT
+
+
+@pytest.mark.parametrize("shape", [(7,), (4, 5), (3, 4, 5)])
+def test_packed_view_bytes_are_the_views(shape):
+    torch = pytest.importorskip("torch")
+    for name in abi._TORCH_DTYPES:
+        t = torch.zeros(shape, dtype=getattr(torch, name.split(".")[1]))
+        for v in (t, t.T if len(shape) == 2 else t[::2], t[..., :0]):
+            assert abi.torch_view_bytes(v) == bytes(abi.torch_view(v)), (name, v.shape)
+    for bad in (torch.zeros((1, 1, 1, 1)), torch.zeros(())):
+        with pytest.raises(ValueError):
+            abi.torch_view_bytes(bad)
+    with pytest.raises(TypeError):
+        abi.torch_view_bytes(torch.zeros(shape, dtype=torch.complex64))
