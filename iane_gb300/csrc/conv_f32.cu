@@ -23,14 +23,16 @@ int launch_conv_f32_tiled(const DevView& src, const DevView& kernel, const DevVi
 		if (rows != IANE_GB_UNSUPPORTED) return rows;
 	}
 	// Small single-plane jobs (too few 64x64 tiles for every SM, and under 5e7 tap-products):
-	// the one-warp blocks of 32x32 tiles are latency-bound there, and the generic kernel (one
-	// output per thread, 256-thread blocks, FP32 sums) with many times the warps per SM is
-	// faster -- measured on GB300: 512^2 7x7 16.5 -> 9.9 us, 256^2 15x15 27.8 -> 8.9 us,
-	// 384x640 11x11 23.5 -> 14.4 us; 1024^2 9x9 (8.5e7) and 512^2 31x31 stay tiled.
+	// the one-warp blocks of 32x32 tiles are latency-bound there, and two outputs per thread in
+	// 256-thread blocks (conv_small.cu) with many times the warps per SM are faster -- measured on
+	// GB300, tiled against one output per thread: 512^2 7x7 16.5 -> 9.9 us, 256^2 15x15 27.8 -> 8.9
+	// us, 384x640 11x11 23.5 -> 14.4 us; two per thread 5.8, 6.2 and 8.7 us; 1024^2 9x9 (8.5e7) and
+	// 512^2 31x31 stay tiled. The smallest jobs stay with one output per thread, which spreads them
+	// over twice the blocks (333x200 3x3: 4.2 us, two per thread 4.4).
 	const long long big_tiles = static_cast<long long>((src.ext[0] + 63) / 64) * ((src.ext[1] + 63) / 64) * src.ext[2];
 	const double work = static_cast<double>(element_count(src)) * kx * ky;
 	if (kz == 1 && big_tiles < 2LL * device_sm_count() && work < 5e7) {
-		return IANE_GB_UNSUPPORTED;
+		return work < 2e6 ? IANE_GB_UNSUPPORTED : launch_conv_small(src, kernel, dst, border, stream, tex);
 	}
 	// Shared memory holds one or two kernel planes' taps (ky x 32 floats at most) next to the
 	// halo tiles; the planes stream through it, so kz has no limit here.

@@ -53,6 +53,11 @@ int convolve_checked(const DevView& s, const DevView& k, const DevView& d, int b
 int launch_conv_f32_tiled(const DevView& src, const DevView& kernel, const DevView& dst, int border,
 	cudaStream_t stream, const TexSource* tex = nullptr);
 
+// Small single-plane FP32 jobs (conv_small.cu), any source type or texture; the generic kernel's
+// bits. IANE_GB_UNSUPPORTED without an error for kernels wider than 31 or taller than 63.
+int launch_conv_small(const DevView& src, const DevView& kernel, const DevView& dst, int border, cudaStream_t stream,
+	const TexSource* tex);
+
 // Row-strip direct FP32 convolution of large 2-D f32 images (or stacks of 2-D planes under a
 // kernel one plane deep) with kernels of odd extents up to 7, line filters included
 // (direct_rows.cu); the same bits as the tiled kernel. IANE_GB_UNSUPPORTED without an error

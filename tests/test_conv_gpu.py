@@ -317,3 +317,27 @@ def test_fft_rejects_integer_types_and_exact_mode(cuda):
     kf = to_gpu(np.ones((3, 3), np.float32))
     with pytest.raises(iane_gb300.IaneInvalidArgument):
         iane_gb300.convolve(f, kf, f.clone(), "zero", exact=True, method="fft")
+
+
+@pytest.mark.parametrize("shape,kshape", [
+    ((257, 259), (7, 7)),     # a column and a row beyond whole blocks
+    ((16, 2080), (63, 1)),    # one block row, the tallest kernel
+    ((1030, 33), (3, 31)),    # a column of one output, the widest kernel
+    ((3, 90, 95), (1, 9, 11)),  # a stack of planes
+])
+@pytest.mark.parametrize("dtype", [np.float32, np.uint8, np.int16], ids=lambda d: np.dtype(d).name)
+@pytest.mark.parametrize("border", ["clamp", "zero", "mirror"])
+def test_small_jobs(cuda, shape, kshape, dtype, border):
+    rng = np.random.default_rng(sum(shape) + sum(kshape))
+    big = (rng.random((*shape[:-1], shape[-1] + 3)) * 200).astype(dtype)
+    kernel = rng.standard_normal(kshape).astype(np.float32)
+    src = np.ascontiguousarray(big[..., 1:-2])
+    ref = np.zeros(shape, np.float32)
+    oracle.convolve(src, kernel, ref, border)
+    scale = magnitude(src, kernel, border)
+    packed, crop = empty_like_np(shape, np.float32), empty_like_np(shape, np.float32)
+    iane_gb300.convolve(to_gpu(src), to_gpu(kernel), packed, border)
+    iane_gb300.convolve(to_gpu(big)[..., 1:-2], to_gpu(kernel), crop, border)
+    got = to_host(packed)
+    assert np.all(np.abs(got.astype(np.float64) - ref) <= 1e-5 * scale + 1e-30)
+    assert np.array_equal(got, to_host(crop))
