@@ -431,6 +431,12 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src, int src_by
 	asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(src_bytes)
 		: "memory");
 }
+// The same for 16 bytes (both addresses 16-byte aligned).
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int src_bytes)
+{
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(src_bytes)
+		: "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template<int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 

@@ -80,6 +80,11 @@ int launch_separable_rows(const DevView& src, const DevView* taps, const DevView
 int launch_morph_planes(const DevView& src, const DevView& dst, const int* radius, bool dilate, int border,
 	cudaStream_t stream);
 
+// Cube erosion / dilation of 3-D f32 volumes with radius 1..3 (morphology_march.cu);
+// IANE_GB_UNSUPPORTED without an error when it does not apply.
+int launch_morph_march(const DevView& src, const DevView& dst, const int* radius, bool dilate, int border,
+	cudaStream_t stream);
+
 // Fused separable FP32 convolution, any tap length (separable.cu).
 int launch_conv_separable(const DevView& src, const DevView* taps, const DevView& dst, int border,
 	cudaStream_t stream);

@@ -416,6 +416,8 @@ int launch_op(const DevView& s, const DevView& d, const int* r, const uint8_t* m
 	}
 	const int planes = launch_morph_planes(s, d, r, DILATE, border, st);
 	if (planes != IANE_GB_UNSUPPORTED) return planes;
+	const int march = launch_morph_march(s, d, r, DILATE, border, st);
+	if (march != IANE_GB_UNSUPPORTED) return march;
 	const size_t smem = box_xy_smem(r[0], r[1], sizeof(T));
 	if (smem > 200 * 1024) {
 		morph_direct_kernel<T, DILATE><<<g8, dim3(32, 8), 0, st>>>(s, d, r[0], r[1], r[2], nullptr, border);

@@ -209,3 +209,33 @@ def test_planes_of_packed_rows(cuda, dtype, shape, radius):
             got = to_host(out)
             assert np.ascontiguousarray(got[..., 1:-1]).tobytes() == ref.tobytes(), (op, border, "crop")
             assert not got[..., 0].any() and not got[..., -1].any()
+
+
+@pytest.mark.parametrize("shape,radius", [
+    ((5, 16, 16), 2), ((1, 17, 20), 1),       # one warp; one plane, a row beyond whole groups of rows
+    ((9, 33, 260), 2), ((40, 20, 128), 1),    # a third warp of one group; several chunks of planes
+    ((17, 120, 132), 3), ((33, 64, 130), 3),  # the widest window; rows that TMA cannot address
+])
+def test_volumes_of_aligned_rows(cuda, shape, radius):
+    # NaN, infinities and zeros of both signs: a warp takes the exact form in planes that hold a -0
+    rng = np.random.default_rng(sum(shape) + radius)
+    src = rng.standard_normal(shape).astype(np.float32)
+    for value in (np.nan, np.inf, -np.inf, 0.0):
+        src[rng.random(shape) < 0.03] = value
+    half = src.copy()
+    src[rng.random(shape) < 0.03] = -0.0
+    half[:1 + shape[0] // 2][rng.random((1 + shape[0] // 2, *shape[1:])) < 0.1] = -0.0  # planes with and without
+    half = np.where(np.abs(half) < 1.0, np.copysign(np.float32(0), half), half)
+    wide = np.zeros((*shape[:-1], shape[-1] + 8), np.float32)
+    for data in (src, half):
+        wide[..., 4:-4] = data
+        for op in ("erode", "dilate"):
+            for border in ("clamp", "zero", "mirror"):
+                ref = np.zeros_like(data)
+                oracle.morphology(data, ref, (radius,) * 3, op, border)
+                assert run_gpu(data, (radius,) * 3, op, border).tobytes() == ref.tobytes(), (op, border)
+                out = to_gpu(np.zeros((*shape[:-1], shape[-1] + 1), np.float32))
+                iane_gb300.morphology(to_gpu(wide)[..., 4:-4], out[..., 1:], (radius,) * 3, op, border)
+                got = to_host(out)
+                assert np.ascontiguousarray(got[..., 1:]).tobytes() == ref.tobytes(), (op, border, "crop")
+                assert not got[..., 0].any()
