@@ -555,7 +555,7 @@ int launch_radius(const DevView& src, const DevView* taps, const DevView& dst, i
 		a.tap_stride[axis] = taps[axis].stride[0];
 		a.k[axis] = taps[axis].ext[0];
 	}
-	const bool z3 = src.ext[2] > 1 || taps[2].ext[0] > 1;
+	const bool z3 = src.rank > 2; // also of one plane: its tap along z counts
 	// TMA wants positive, 16-byte multiple pitches that do not make rows or planes overlap.
 	a.use_tma = (rows_aligned16(src) && (src.ext[1] <= 1 || src.stride[1] >= 4LL * src.ext[0]) &&
 		(src.ext[2] <= 1 || (src.stride[2] > 0 && src.stride[2] >= (src.ext[1] > 1 ? src.stride[1] : 4LL * src.ext[0]) *

@@ -226,7 +226,7 @@ int launch_separable_rows(const DevView& src, const DevView* taps, const DevView
 {
 	int r = 0;
 	for (int i = 0; i < 2; ++i) r = max(r, taps[i].ext[0] / 2);
-	const bool two_d = src.rank <= 2 || (src.ext[2] == 1 && taps[2].ext[0] == 1);
+	const bool two_d = src.rank <= 2; // one plane of a volume still has its tap along z
 	// large images only (from 4 M pixels: smaller ones are launch-bound and take the tiled
 	// kernel; the border rules also assume a strip's width and four steps of rows), f32 rows TMA
 	// can address, radius <= 7 on both axes

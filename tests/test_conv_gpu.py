@@ -206,6 +206,19 @@ def test_separable_parity(cuda, shape, taps, border):
     assert float(np.max(np.abs(out - ref) / np.maximum(np.abs(ref), 1e-30))) <= FP32_TOL
 
 
+@pytest.mark.parametrize("shape", [(1, 17, 20), (1, 5, 7), (1, 600, 640)])
+def test_separable_one_plane_single_tap(cuda, shape):
+    # one plane under a single tap along z that is not 1
+    rng = np.random.default_rng(sum(shape))
+    src = rng.random(shape, dtype=np.float32) + np.float32(0.01)
+    tap_list = [gaussian((3,), (1.0,)), gaussian((3,), (1.0,)), np.float32([0.75])]
+    ref = np.zeros_like(src)
+    oracle.convolve_separable(src, tap_list, ref, "clamp")
+    d = empty_like_np(shape, np.float32)
+    iane_gb300.convolve_separable(to_gpu(src), [to_gpu(t) for t in tap_list], d, "clamp")
+    assert float(np.max(np.abs(to_host(d) - ref) / ref)) <= (7 + 6) * 2.0 ** -24
+
+
 def test_separable_strided_views(cuda):
     t = torch()
     rng = np.random.default_rng(8)
