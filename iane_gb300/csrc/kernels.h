@@ -70,6 +70,11 @@ int launch_direct_rows(const DevView& src, const DevView& kernel, const DevView&
 int launch_conv_separable_fast(const DevView& src, const DevView* taps, const DevView& dst, int border,
 	cudaStream_t stream);
 
+// 3-D f32 volumes with TMA-addressable rows, radii r <= 4 (separable_march.cu);
+// IANE_GB_UNSUPPORTED without an error when it does not apply.
+int launch_separable_march(const DevView& src, const DevView* taps, const DevView& dst, int border, int r,
+	cudaStream_t stream);
+
 // Large 2-D f32 images (separable_rows.cu): IANE_GB_UNSUPPORTED when the view or radius does
 // not qualify.
 int launch_separable_rows(const DevView& src, const DevView* taps, const DevView& dst, int border,

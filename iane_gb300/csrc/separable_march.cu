@@ -1,0 +1,204 @@
+// Separable FP32 convolution of 3-D f32 volumes (up to nine taps per axis): warps that march down z
+// on their own, as morphology_march.cu does.
+//
+// What bounds it: memory (8 B per voxel) and the FMA issue next to it. A block-wide kernel
+// that passes every plane through shared memory three times, with two block barriers
+// per pair of planes, waits at them: issue 59%, DRAM 41% of what they can. Here a lane owns 4
+// columns and 4 rows: it takes its rows and their neighbours from the warp's ring of input planes
+// (warp_ring.cuh, TMA two planes ahead), filters each row along x, the columns along y, and adds
+// the result to the 2 R unfinished outputs of every voxel along z, all in registers. The y and z
+// sums are packed two columns to an instruction, taps in pairs from shared memory.
+// Mirror border, that kernel -> here: 512^3 3 taps 199 -> 176 us, 5 taps 255 -> 175 (90% of the
+// measured HBM rate), 7 taps 306 -> 246, 9 taps 401 -> 305; 256 x 256 x 64 7 taps 21.6 -> 18.6.
+//
+// Rounding points are those of successive 1-D convolutions with an f32 intermediate; x and y sums
+// run from tap 0 up, the z sums from the oldest plane to the newest.
+#include "kernels.h"
+#include "warp_ring.cuh"
+
+namespace iane_gb {
+namespace {
+
+constexpr int OUT = kRingOut;
+constexpr int WARPS = 4;            // warps of a block, one above the other
+
+struct MarchArgs {
+	RingArgs in;
+	char* dst;
+	long long d_stride[3];    // bytes
+	int zc;                   // output planes of a block
+	int dst16;                // destination rows contiguous and 16-byte aligned
+	const char* tap_ptr[3];   // 1-D f32 device views of the taps (null: axis beyond the rank)
+	long long tap_stride[3];
+	int k[3];
+};
+
+template<int R, bool EDGE>
+__device__ __forceinline__ void filter_rows(const WarpRing<R>& ring, const float4* plane, const float (&tx)[2 * R + 1],
+	float2 (&h)[OUT + 2 * R][OUT / 2])
+{
+#pragma unroll
+	for (int r = 0; r < OUT + 2 * R; ++r) {
+		float w[OUT + 2 * R], o[OUT];
+		ring.template row<EDGE>(plane, r, w);
+#pragma unroll
+		for (int i = 0; i < OUT; ++i) {
+			float s = 0.0f;
+#pragma unroll
+			for (int q = 0; q <= 2 * R; ++q) s = fmaf(tx[q], w[i + 2 * R - q], s);
+			o[i] = s;
+		}
+#pragma unroll
+		for (int p = 0; p < OUT / 2; ++p) h[r][p] = make_float2(o[2 * p], o[2 * p + 1]);
+	}
+}
+
+template<int R>
+__global__ void __launch_bounds__(32 * WARPS, R >= 3 ? 2 : R == 2 ? 3 : 4)
+	separable_march_kernel(const __grid_constant__ CUtensorMap map, const MarchArgs a)
+{
+	constexpr int K = 2 * R + 1;
+	constexpr int ROWS = OUT + 2 * R;
+	constexpr int PAIRS = OUT / 2;
+	extern __shared__ __align__(128) unsigned char smem[];
+	__shared__ float2 taps[2][K]; // (t, t) of axes 1 and 2
+	const int lane = threadIdx.x, warp = threadIdx.y;
+	const int nx = a.in.nx, ny = a.in.ny;
+	const int xw = blockIdx.x * kRingColumns;
+	const int x = xw + OUT * lane;
+	const int y0 = (blockIdx.y * WARPS + warp) * OUT;
+	const int z0 = blockIdx.z * a.zc, z1 = min(a.in.nz, z0 + a.zc);
+
+	// taps centred and zero-padded to 2 R + 1; an axis beyond the rank is the single tap 1
+	auto tap = [&](int axis, int i) -> float {
+		if (!a.tap_ptr[axis]) return i == R ? 1.0f : 0.0f;
+		const int q = i - (R - a.k[axis] / 2);
+		return q >= 0 && q < a.k[axis] ? *reinterpret_cast<const float*>(a.tap_ptr[axis] + q * a.tap_stride[axis]) : 0.0f;
+	};
+	float tx[K];
+#pragma unroll
+	for (int i = 0; i < K; ++i) tx[i] = tap(0, i);
+	const int tid = warp * 32 + lane;
+	if (tid < 2 * K) {
+		const float t = tap(1 + tid / K, tid % K);
+		taps[tid / K][tid % K] = make_float2(t, t);
+	}
+	__syncthreads();
+	if (y0 >= ny) return;
+	WarpRing<R> ring;
+	ring.begin(smem, WARPS, warp, &map, a.in, xw, y0, z0 - R, z1 + R);
+	const bool whole = x + OUT <= nx;
+	char* const column = a.dst + x * a.d_stride[0] + y0 * a.d_stride[1];
+
+	// unfinished outputs: pending[k] has met its first 2 R - k planes
+	float2 pending[2 * R][OUT][PAIRS];
+#pragma unroll
+	for (int k = 0; k < 2 * R; ++k)
+#pragma unroll
+		for (int j = 0; j < OUT; ++j)
+#pragma unroll
+			for (int p = 0; p < PAIRS; ++p) pending[k][j][p] = make_float2(0.0f, 0.0f);
+
+	for (int z = z0 - R; z < z1 + R; ++z) {
+		const float4* plane = ring.plane(&map, a.in, z);
+		float2 h[ROWS][PAIRS]; // every row filtered along x
+		if (ring.edge) {
+			filter_rows<R, true>(ring, plane, tx, h);
+		} else {
+			filter_rows<R, false>(ring, plane, tx, h);
+		}
+		if (z + 1 < z1 + R) ring.prepare(a.in);
+		float2 m[OUT][PAIRS];
+#pragma unroll
+		for (int j = 0; j < OUT; ++j)
+#pragma unroll
+			for (int p = 0; p < PAIRS; ++p) m[j][p] = make_float2(0.0f, 0.0f);
+#pragma unroll
+		for (int q = 0; q < K; ++q) {
+			const float2 t = taps[0][q];
+#pragma unroll
+			for (int j = 0; j < OUT; ++j)
+#pragma unroll
+				for (int p = 0; p < PAIRS; ++p) m[j][p] = __ffma2_rn(h[j + 2 * R - q][p], t, m[j][p]);
+		}
+		// input plane z meets tap q of output z - R + q: it completes the oldest and joins the others
+		const int zo = z - R;
+		if (zo >= z0) {
+			const float2 t = taps[1][0];
+			char* out = column + zo * a.d_stride[2];
+#pragma unroll
+			for (int j = 0; j < OUT; ++j) {
+				if (y0 + j >= ny) break;
+				float2 o[PAIRS];
+#pragma unroll
+				for (int p = 0; p < PAIRS; ++p) o[p] = __ffma2_rn(m[j][p], t, pending[0][j][p]);
+				char* row = out + j * a.d_stride[1];
+				if (a.dst16 && whole) {
+					*reinterpret_cast<float4*>(row) = make_float4(o[0].x, o[0].y, o[1].x, o[1].y);
+				} else {
+					const float v[OUT] = {o[0].x, o[0].y, o[1].x, o[1].y};
+#pragma unroll
+					for (int i = 0; i < OUT; ++i) {
+						if (x + i < nx) *reinterpret_cast<float*>(row + i * a.d_stride[0]) = v[i];
+					}
+				}
+			}
+		}
+#pragma unroll
+		for (int k = 0; k < 2 * R; ++k) {
+			const float2 t = taps[1][k + 1];
+#pragma unroll
+			for (int j = 0; j < OUT; ++j)
+#pragma unroll
+				for (int p = 0; p < PAIRS; ++p) {
+					const float2 seen = k + 1 < 2 * R ? pending[k + 1 < 2 * R ? k + 1 : 0][j][p] : make_float2(0.0f, 0.0f);
+					pending[k][j][p] = __ffma2_rn(m[j][p], t, seen);
+				}
+		}
+	}
+}
+
+template<int R>
+int launch(const DevView& s, MarchArgs a, cudaStream_t st)
+{
+	constexpr size_t smem = WarpRing<R>::bytes(WARPS);
+	auto kernel = separable_march_kernel<R>;
+	IANE_GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+		"separable: set shared memory size");
+	CUtensorMap map{};
+	const int status = ring_map<R>(&map, s);
+	if (status) return status;
+	const dim3 tiles((a.in.nx + kRingColumns - 1) / kRingColumns, (a.in.ny + OUT * WARPS - 1) / (OUT * WARPS));
+	a.zc = ring_chunk(static_cast<long long>(tiles.x) * tiles.y, a.in.nz, R,
+		static_cast<long long>(R >= 3 ? 2 : R == 2 ? 3 : 4) * device_sm_count());
+	kernel<<<dim3(tiles.x, tiles.y, (a.in.nz + a.zc - 1) / a.zc), dim3(32, WARPS), smem, st>>>(map, a);
+	IANE_GB_CUDA(cudaGetLastError(), "separable: launch");
+	return IANE_GB_OK;
+}
+
+}  // namespace
+
+int launch_separable_march(const DevView& src, const DevView* taps, const DevView& dst, int border, int r, cudaStream_t st)
+{
+	if (!ring_supported(src) || r > 4) return IANE_GB_UNSUPPORTED;
+	MarchArgs a{};
+	a.in = RingArgs{src.ext[0], src.ext[1], src.ext[2], border, device_status_ptr()};
+	if (!a.in.status) return IANE_GB_CUDA_ERROR;
+	a.dst = dst.ptr;
+	for (int i = 0; i < 3; ++i) a.d_stride[i] = dst.stride[i];
+	a.dst16 = rows_aligned16(dst) ? 1 : 0;
+	for (int axis = 0; axis < 3; ++axis) {
+		a.tap_ptr[axis] = taps[axis].ptr;
+		a.tap_stride[axis] = taps[axis].stride[0];
+		a.k[axis] = taps[axis].ext[0];
+	}
+	switch (r) {
+	case 0:
+	case 1: return launch<1>(src, a, st);
+	case 2: return launch<2>(src, a, st);
+	case 3: return launch<3>(src, a, st);
+	default: return launch<4>(src, a, st);
+	}
+}
+
+}  // namespace iane_gb

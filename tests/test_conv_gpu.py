@@ -219,6 +219,35 @@ def test_separable_one_plane_single_tap(cuda, shape):
     assert float(np.max(np.abs(to_host(d) - ref) / ref)) <= (7 + 6) * 2.0 ** -24
 
 
+@pytest.mark.parametrize("shape,taps", [
+    ((5, 16, 16), (3, 1, 3)), ((1, 17, 20), (3, 3, 1)),    # one warp; one plane under three taps
+    ((9, 33, 260), (5, 3, 5)), ((40, 20, 128), (1, 5, 3)),  # a third warp of one group; several chunks of planes
+    ((17, 120, 132), (7, 7, 5)), ((33, 64, 130), (9, 7, 9)), ((6, 19, 131), (9, 9, 9)),
+])
+def test_separable_volumes(cuda, shape, taps):
+    # contiguous, and inside a wider volume whose rows TMA can address, with results beside its alignment
+    # and with a stride along every axis
+    rng = np.random.default_rng(sum(shape) + sum(taps))
+    src = rng.random(shape, dtype=np.float32) + np.float32(0.01)
+    tap_list = [rng.random(n, dtype=np.float32) + np.float32(0.1) for n in taps]
+    # positive data and taps: n products and n sums per pass, and the oracle's own rounding to f32 per pass
+    tol = (sum(taps) + 6) * 2.0 ** -24
+    pad = 8 + -shape[-1] % 4
+    wide = np.full((*shape[:-1], shape[-1] + pad), 7, np.float32)
+    wide[..., 4:4 + shape[-1]] = src
+    taps_gpu = [to_gpu(t) for t in tap_list]
+    for border in ("clamp", "zero", "mirror"):
+        ref = np.zeros_like(src)
+        oracle.convolve_separable(src, tap_list, ref, border)
+        for g in (to_gpu(src), to_gpu(wide)[..., 4:4 + shape[-1]]):
+            aside = torch().zeros((*shape[:-1], shape[-1] + 1), device="cuda")
+            apart = torch().zeros((*shape[:-1], 2 * shape[-1]), device="cuda")
+            for out in (torch().zeros(shape, device="cuda"), aside[..., 1:], apart[..., ::2]):
+                iane_gb300.convolve_separable(g, taps_gpu, out, border)
+                assert float(np.max(np.abs(to_host(out) - ref) / ref)) <= tol, border
+            assert not to_host(aside)[..., 0].any() and not to_host(apart)[..., 1::2].any()
+
+
 def test_separable_strided_views(cuda):
     t = torch()
     rng = np.random.default_rng(8)
