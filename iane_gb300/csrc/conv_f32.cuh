@@ -57,9 +57,24 @@ int launch_f32_kx(const DevView& src, const DevView& kernel, const DevView& dst,
 	}
 	// single-plane kernels on large images: direct summation (fewer registers, more blocks)
 	const bool single = big && a.kz == 1;
+	// 3-D kernels up to 15 wide take 16 x 2 outputs per lane: fewer kernel-row loads and checks
+	// per FMA, the same sums. Wider ones keep 8 x 4, whose row segment needs fewer registers,
+	// and so do single-plane kernels: 16 x 2 costs them the seventh block per SM, and held to
+	// 72 registers it still measured slower (8192^2 7x7 mirror: 0.166 -> 0.176 / 0.192 ms).
+	constexpr int RX = KX <= 15 ? 16 : kRX, RY = KX <= 15 ? 2 : kRY;
+	// 16 x 2 has four blocks per SM. Where the tiles need a second wave for at most one block per SM
+	// more, 8 x 4 held to five blocks takes them in one, for kernels up to 9 wide (253 x 187 x 61, 732
+	// tiles, 7 x 7 x 5, four per SM -> five: by copies 76 -> 61 us, by TMA 64 -> 55; 9 x 9 x 5 91 -> 77,
+	// 80 -> 77; 13 x 13 x 5 144 -> 172). Just above four (612 tiles) it still pays with copies (65 ->
+	// 60), by TMA no longer (50 -> 54).
+	const bool five = KX <= 9 && big && !single && 2 * big_tiles > (stage == kTileTma ? 9LL : 8LL) * device_sm_count() &&
+		big_tiles <= 5LL * device_sm_count();
 	if (stage == kTileCopy) {
-		return single ? launch_tile<KX, 2, 2, kTileCopy, true>(map, a, epi, stream)
-			: big ? launch_tile<KX, 2, 2, kTileCopy>(map, a, epi, stream)
+		// up to 15 wide held to seven blocks per SM, as TMA staging has them by itself (2047 x 2049 bf16
+		// 9 x 9 mirror: 41 -> 33 us)
+		return single ? launch_tile<KX, 2, 2, kTileCopy, true, kRX, kRY, KX <= 15 ? 7 : 0>(map, a, epi, stream)
+			: five ? launch_tile<KX, 2, 2, kTileCopy, false, kRX, kRY, KX <= 9 ? 5 : 0>(map, a, epi, stream)
+			: big ? launch_tile<KX, 2, 2, kTileCopy, false, RX, RY>(map, a, epi, stream)
 			: launch_tile<KX, 1, 1, kTileCopy>(map, a, epi, stream);
 	}
 	// box = one halo tile at the shared-memory pitch (f32) or the raw narrow box
@@ -72,12 +87,8 @@ int launch_f32_kx(const DevView& src, const DevView& kernel, const DevView& dst,
 		const int status =
 			encode_tensor_map_f32(&map, src.ptr, src.ext[0], src.ext[1], src.ext[2], row, plane, box_w, box_h);
 		if (status) return status;
-		// 3-D kernels up to 15 wide take 16 x 2 outputs per lane: fewer kernel-row loads and checks
-		// per FMA, the same sums. Wider ones keep 8 x 4, whose row segment needs fewer registers,
-		// and so do single-plane kernels: 16 x 2 costs them the seventh block per SM, and held to
-		// 72 registers it still measured slower (8192^2 7x7 mirror: 0.166 -> 0.176 / 0.192 ms).
-		constexpr int RX = KX <= 15 ? 16 : kRX, RY = KX <= 15 ? 2 : kRY;
 		return single ? launch_tile<KX, 2, 2, kTileTma, true>(map, a, epi, stream)
+			: five ? launch_tile<KX, 2, 2, kTileTma, false, kRX, kRY, KX <= 9 ? 5 : 0>(map, a, epi, stream)
 			: big ? launch_tile<KX, 2, 2, kTileTma, false, RX, RY>(map, a, epi, stream)
 			: launch_tile<KX, 1, 1, kTileTma>(map, a, epi, stream);
 	}

@@ -122,61 +122,111 @@ inline size_t tile_smem_bytes(int ky, int kz, int stage = kTileCopy, int esize =
 	return base + 16;
 }
 
-// Element-by-element staging for element types other than f32 and for textures: batches of
-// loads are issued before any is stored so that their latencies overlap; integer and bf16
-// elements are loaded raw by size and converted afterwards.
+// Element-by-element staging deals whole rows to the warps: the border rule is applied once per row and
+// once per column and thread, not per cell (with the divisions of a flat cell number it cost as many
+// instructions as the sums: 2557 x 1917 9 x 9 u8 clamp 62 -> 50 us, 5 x 5 u16 mirror 48 -> 35, 21 x 21
+// f32 zero 101 -> 88; 253 x 187 x 61 f32, 7 x 7 x 5, 78 -> 61 with the five blocks of conv_f32.cuh).
+template<int W>
+struct StageColumns {
+	static constexpr int N = (W + 31) / 32; // of a thread: lane, lane + 32, ...
+	int xi[N];
+	uint32_t in = 0; // bit c: column c lies in the image (else the zero value)
+
+	__device__ __forceinline__ StageColumns(const TileArgs& a, int gx0)
+	{
+#pragma unroll
+		for (int c = 0; c < N; ++c) {
+			const int col = (threadIdx.x & 31) + 32 * c;
+			xi[c] = 0;
+			if (map_coord(gx0 + col, a.nx, a.border, xi[c])) in |= 1u << c;
+		}
+	}
+	static __device__ __forceinline__ bool has(int c) { return static_cast<int>(threadIdx.x & 31) + 32 * c < W; }
+};
+
+// f32 elements by 4-byte cp.async.
+template<int W, int P, int NT>
+__device__ __forceinline__ void stage_f32(const TileArgs& a, float* dst, int gx0, int gy0, int H, int zi, bool zok)
+{
+	constexpr int N = StageColumns<W>::N;
+	const StageColumns<W> cols(a, gx0);
+	long long xo[N]; // of a column outside a zero border: 0, and no bytes are read
+	int bytes[N];
+#pragma unroll
+	for (int c = 0; c < N; ++c) {
+		xo[c] = cols.xi[c] * a.s_stride[0];
+		bytes[c] = zok && (cols.in & (1u << c)) ? 4 : 0;
+	}
+	const char* plane = a.src + zi * a.s_stride[2];
+	float* to = dst + (threadIdx.x >> 5) * P + (threadIdx.x & 31);
+	for (int r = threadIdx.x >> 5; r < H; r += NT / 32, to += NT / 32 * P) {
+		int yi = 0;
+		const bool ok = map_coord(gy0 + r, a.ny, a.border, yi);
+		const char* row = plane + yi * a.s_stride[1];
+#pragma unroll
+		for (int c = 0; c < N; ++c) {
+			if (StageColumns<W>::has(c)) cp_async4(to + 32 * c, row + xo[c], ok ? bytes[c] : 0);
+		}
+	}
+}
+
+// Other element types and textures: batches of loads are issued before any is stored so that their
+// latencies overlap; integer and bf16 elements are loaded raw by size and converted afterwards.
 template<int W, int P, int NT>
 __device__ __forceinline__ void stage_elements(const TileArgs& a, float* dst, int gx0, int gy0, int H, int zi, bool zok)
 {
-	constexpr int kBatch = 8;
-	const int tid = threadIdx.x;
-	const int n = W * H;
+	constexpr int N = StageColumns<W>::N;
+	constexpr int ROWS = N >= 3 ? 3 : 4; // of a batch
+	constexpr int WARPS = NT / 32;
+	const StageColumns<W> cols(a, gx0);
+	const int lane = threadIdx.x & 31;
 	const char* plane = a.src + zi * a.s_stride[2];
 	const bool texture = a.stage == kStageTexture;
 	const int esize = a.src_dtype == IANE_GB_U8 || a.src_dtype == IANE_GB_I8 ? 1 :
 		(a.src_dtype == IANE_GB_U16 || a.src_dtype == IANE_GB_I16 || a.src_dtype == IANE_GB_BF16 ? 2 : 4);
-	for (int base = tid; base < n; base += NT * kBatch) {
-		uint32_t raw[kBatch]; // element bits, or a texel's float bits
-		uint32_t in = 0;      // bit u: sample u lies in the image (else it is the zero value)
+	for (int base = threadIdx.x >> 5; base < H; base += WARPS * ROWS) {
+		uint32_t raw[ROWS][N]; // element bits, or a texel's float bits
+		uint32_t in[ROWS];     // as StageColumns::in
 #pragma unroll
-		for (int u = 0; u < kBatch; ++u) {
-			const int i = base + u * NT;
-			raw[u] = 0;
-			if (i < n) {
-				const int r = i / W, c = i - (i / W) * W;
-				int xi = 0, yi = 0;
-				if (zok && map_coord(gx0 + c, a.nx, a.border, xi) && map_coord(gy0 + r, a.ny, a.border, yi)) {
-					in |= 1u << u;
-					if (texture) {
-						raw[u] = __float_as_uint(texel_as_float(a.tex.tex, a.tex.dtype, a.tex.rank, a.tex.origin[0] + xi,
-							a.tex.origin[1] + yi, a.tex.origin[2] + zi));
-					} else {
-						const char* q = plane + xi * a.s_stride[0] + yi * a.s_stride[1];
-						raw[u] = esize == 1 ? static_cast<uint32_t>(*reinterpret_cast<const uint8_t*>(q))
-							: esize == 2 ? static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(q))
-							: *reinterpret_cast<const uint32_t*>(q);
-					}
+		for (int u = 0; u < ROWS; ++u) {
+			const int r = base + u * WARPS;
+			int yi = 0;
+			in[u] = r < H && zok && map_coord(gy0 + r, a.ny, a.border, yi) ? cols.in : 0u;
+			const char* row = plane + yi * a.s_stride[1];
+#pragma unroll
+			for (int c = 0; c < N; ++c) { // without branches, so that all are in flight: cells outside read the image's first
+				if (texture) {
+					raw[u][c] = __float_as_uint(texel_as_float(a.tex.tex, a.tex.dtype, a.tex.rank, a.tex.origin[0] + cols.xi[c],
+						a.tex.origin[1] + yi, a.tex.origin[2] + zi));
+				} else {
+					const char* q = row + cols.xi[c] * a.s_stride[0];
+					raw[u][c] = esize == 1 ? static_cast<uint32_t>(*reinterpret_cast<const uint8_t*>(q))
+						: esize == 2 ? static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(q))
+						: *reinterpret_cast<const uint32_t*>(q);
 				}
 			}
 		}
 #pragma unroll
-		for (int u = 0; u < kBatch; ++u) {
-			const int i = base + u * NT;
-			if (i >= n) break;
-			float v = 0.0f;
-			if (in & (1u << u)) {
-				const int dt = texture ? IANE_GB_F32 : a.src_dtype;
-				switch (dt) {
-				case IANE_GB_U8: case IANE_GB_U16: case IANE_GB_U32: v = static_cast<float>(raw[u]); break;
-				case IANE_GB_I8: v = static_cast<float>(static_cast<int8_t>(raw[u])); break;
-				case IANE_GB_I16: v = static_cast<float>(static_cast<int16_t>(raw[u])); break;
-				case IANE_GB_I32: v = static_cast<float>(static_cast<int32_t>(raw[u])); break;
-				case IANE_GB_BF16: v = __uint_as_float(raw[u] << 16); break;
-				default: v = __uint_as_float(raw[u]); break; // f32 bits
+		for (int u = 0; u < ROWS; ++u) {
+			const int r = base + u * WARPS;
+			if (r >= H) break;
+#pragma unroll
+			for (int c = 0; c < N; ++c) {
+				if (!StageColumns<W>::has(c)) continue;
+				float v = 0.0f;
+				if (in[u] & (1u << c)) {
+					const uint32_t bits = raw[u][c];
+					switch (texture ? IANE_GB_F32 : a.src_dtype) {
+					case IANE_GB_U8: case IANE_GB_U16: case IANE_GB_U32: v = static_cast<float>(bits); break;
+					case IANE_GB_I8: v = static_cast<float>(static_cast<int8_t>(bits)); break;
+					case IANE_GB_I16: v = static_cast<float>(static_cast<int16_t>(bits)); break;
+					case IANE_GB_I32: v = static_cast<float>(static_cast<int32_t>(bits)); break;
+					case IANE_GB_BF16: v = __uint_as_float(bits << 16); break;
+					default: v = __uint_as_float(bits); break; // f32 bits
+					}
 				}
+				dst[r * P + lane + 32 * c] = v;
 			}
-			const int r = i / W, c = i - (i / W) * W;
-			dst[r * P + c] = v;
 		}
 	}
 }
@@ -287,8 +337,11 @@ __device__ __forceinline__ void plane_sums(float (&sum)[RY][RX], const float* ti
 // (bit b for buffer b) from one call to the next, and `bars` are the two tile mbarriers (TMA
 // stages), initialised by the caller. The caller applies its epilogue to acc afterwards, so
 // none of the epilogue's state is live during the sums.
+// FRESH: no call before this one in the block (its buffers are free): the tile comes while the taps do.
+// It pays for single planes (2560 x 1920 u8 9 x 9 clamp 36.9 -> 30.5 us, with the edge fix-up by rows);
+// where several planes follow it does not (64 x 256 x 256 under 15 x 15 x 7: 220.3 -> 222).
 // taps_resident: a single-plane caller's previous call left this kernel's taps in shared memory.
-template<int KX, int WX, int WY, int STAGE, bool SINGLE = false, int RX = kRX, int RY = kRY>
+template<int KX, int WX, int WY, int STAGE, bool SINGLE = false, int RX = kRX, int RY = kRY, bool FRESH = false>
 __device__ __forceinline__ void conv_tile_sums(const CUtensorMap* tmap_ptr, const TileArgs& a, int x0, int y0, int z,
 	uint32_t& phases, uint64_t* bars, float (&acc)[RY][RX], bool taps_resident = false)
 {
@@ -346,9 +399,6 @@ __device__ __forceinline__ void conv_tile_sums(const CUtensorMap* tmap_ptr, cons
 			dst[i] = v;
 		}
 	};
-	if (nplanes > 0 && !(SINGLE && taps_resident)) load_taps(0);
-	if (nplanes > 1) load_taps(1);
-	__syncthreads(); // taps visible; every lane is done with the previous tile's buffers
 
 	auto issue = [&](int p) {
 		float* dst = tiles + (p & 1) * plane_floats;
@@ -372,16 +422,8 @@ __device__ __forceinline__ void conv_tile_sums(const CUtensorMap* tmap_ptr, cons
 		} else {
 			int zi = 0;
 			const bool zok = map_coord(z + rz - qz, a.nz, a.border, zi);
-			const char* plane = a.src + zi * a.s_stride[2];
 			if (a.stage == kStageF32) {
-				for (int i = tid; i < W * H; i += NT) {
-					const int col = i % W, row = i / W;
-					int xi = 0, yi = 0;
-					const bool ok = zok && map_coord(x0 - G::RXA + col, a.nx, a.border, xi) &&
-						map_coord(y0 - ry + row, a.ny, a.border, yi);
-					const char* src = ok ? plane + xi * a.s_stride[0] + yi * a.s_stride[1] : a.src;
-					cp_async4(dst + row * P + col, src, ok ? 4 : 0);
-				}
+				stage_f32<W, P, NT>(a, dst, x0 - G::RXA, y0 - ry, H, zi, zok);
 			} else {
 				// plain loads and stores; the wait and barrier before the tile is read order them
 				stage_elements<W, P, NT>(a, dst, x0 - G::RXA, y0 - ry, H, zi, zok);
@@ -390,6 +432,15 @@ __device__ __forceinline__ void conv_tile_sums(const CUtensorMap* tmap_ptr, cons
 		}
 	};
 
+	auto issue_first = [&] {
+		if (nplanes > 0) issue(0);
+		if (nplanes > 1) issue(1);
+	};
+	if constexpr (FRESH) issue_first();
+	if (nplanes > 0 && !(SINGLE && taps_resident)) load_taps(0);
+	if (nplanes > 1) load_taps(1);
+	__syncthreads(); // taps visible; every lane is done with the previous tile's buffers
+	if constexpr (!FRESH) issue_first();
 
 #pragma unroll
 	for (int j = 0; j < RY; ++j)
@@ -403,8 +454,6 @@ __device__ __forceinline__ void conv_tile_sums(const CUtensorMap* tmap_ptr, cons
 	// nx > rx and ny > ry (the launcher's condition); any other cell keeps the TMA's zeros.
 	const bool fix_tile = STAGE != kTileCopy && a.border != IANE_GB_BORDER_ZERO &&
 		!(x0 - G::RXA >= 0 && x0 - G::RXA + W <= a.nx && y0 - ry >= 0 && y0 + TY + ry <= a.ny);
-	if (nplanes > 0) issue(0);
-	if (nplanes > 1) issue(1);
 	for (int p = 0; p < nplanes; ++p) {
 		if constexpr (STAGE != kTileCopy) {
 			const uint32_t bit = 1u << (p & 1);
@@ -421,18 +470,27 @@ __device__ __forceinline__ void conv_tile_sums(const CUtensorMap* tmap_ptr, cons
 			if (fix_tile) {
 				float* t = tiles + (p & 1) * plane_floats;
 				const int gx0 = x0 - G::RXA, gy0 = y0 - ry;
-				for (int i = tid; i < W * H; i += NT) {
-					const int r = i / W, c = i - r * W;
-					const int gx = gx0 + c, gy = gy0 + r;
-					const int dx = gx < 0 ? -gx : (gx >= a.nx ? gx - a.nx + 1 : 0);
-					const int dy = gy < 0 ? -gy : (gy >= a.ny ? gy - a.ny + 1 : 0);
-					if ((dx == 0 && dy == 0) || dx > G::rx || dy > ry) continue;
-					int mx = 0, my = 0;
-					map_coord(gx, a.nx, a.border, mx);
+				// Whole rows to the warps: the rows' in-image columns are [c0, c1), a lane fixes one beside them.
+				// (Looking at every cell cost an edge tile more than its sums: 256 x 256 x 128 f32 7 x 7 x 5
+				// mirror 229 -> 134 us, 2048^2 9 x 9 25.6 -> 18.2.)
+				const int c0 = max(0, -gx0), c1 = min(W, a.nx - gx0);
+				const int lefts = min(c0, G::rx), fixes = lefts + min(W - c1, G::rx);
+				const int col = lane < lefts ? c0 - lefts + lane : c1 + lane - lefts;
+				int mx = 0;
+				map_coord(gx0 + col, a.nx, a.border, mx);
+				const int from = mx - gx0;
+				const bool beside = lane < fixes && from >= 0 && from < W;
+				for (int r = warp; r < H; r += NT / 32) {
+					const int gy = gy0 + r;
+					if (gy < -ry || gy >= a.ny + ry) continue;
+					int my = 0;
 					map_coord(gy, a.ny, a.border, my);
-					const int lc = mx - gx0, lr = my - gy0;
-					if (lc < 0 || lc >= W || lr < 0 || lr >= H) continue;
-					t[r * P + c] = t[lr * P + lc];
+					const int lr = my - gy0;
+					if (lr < 0 || lr >= H) continue;
+					if (beside) t[r * P + col] = t[lr * P + from];
+					if (lr != r) {
+						for (int c = c0 + lane; c < c1; c += 32) t[r * P + c] = t[lr * P + c];
+					}
 				}
 				__syncthreads(); // fixed tile visible to all lanes
 			}
@@ -495,8 +553,7 @@ __device__ __forceinline__ uint64_t* tile_barriers(int ky, int kz)
 }
 
 template<int KX, int WX, int WY, int STAGE, class Epi, bool SINGLE, int RX, int RY>
-__global__ void __launch_bounds__(32 * WX * WY)
-	conv_tile_kernel(const __grid_constant__ CUtensorMap tmap, const TileArgs a, const __grid_constant__ Epi epi_in)
+__device__ __forceinline__ void conv_tile_block(const CUtensorMap& tmap, const TileArgs& a, const Epi& epi_in)
 {
 	if constexpr (STAGE != kTileCopy) {
 		if (threadIdx.x == 0) {
@@ -509,7 +566,7 @@ __global__ void __launch_bounds__(32 * WX * WY)
 	uint32_t phases = 0;
 	const int x0 = blockIdx.x * 32 * WX, y0 = blockIdx.y * 32 * WY;
 	float acc[RY][RX];
-	conv_tile_sums<KX, WX, WY, STAGE, SINGLE, RX, RY>(&tmap, a, x0, y0, blockIdx.z, phases,
+	conv_tile_sums<KX, WX, WY, STAGE, SINGLE, RX, RY, SINGLE>(&tmap, a, x0, y0, blockIdx.z, phases,
 		tile_barriers<KX, WX, WY>(a.ky, a.kz), acc);
 	// the epilogue's state (pointers, Kahan sums) comes to life only after the sums
 	Epi epi = epi_in;
@@ -522,11 +579,29 @@ __global__ void __launch_bounds__(32 * WX * WY)
 	epi.finish();
 }
 
+template<int KX, int WX, int WY, int STAGE, class Epi, bool SINGLE, int RX, int RY>
+__global__ void __launch_bounds__(32 * WX * WY)
+	conv_tile_kernel(const __grid_constant__ CUtensorMap tmap, const TileArgs a, const __grid_constant__ Epi epi)
+{
+	conv_tile_block<KX, WX, WY, STAGE, Epi, SINGLE, RX, RY>(tmap, a, epi);
+}
+
+// The same held to the registers of BLOCKS blocks per SM.
+template<int KX, int WX, int WY, int STAGE, class Epi, bool SINGLE, int RX, int RY, int BLOCKS>
+__global__ void __launch_bounds__(32 * WX * WY, BLOCKS)
+	conv_tile_kernel_held(const __grid_constant__ CUtensorMap tmap, const TileArgs a, const __grid_constant__ Epi epi)
+{
+	conv_tile_block<KX, WX, WY, STAGE, Epi, SINGLE, RX, RY>(tmap, a, epi);
+}
+
 // Launch helper: grid = tiles over (x, y) and one block per output plane; RX x RY outputs per lane.
-template<int KX, int WX, int WY, int STAGE, bool SINGLE = false, int RX = kRX, int RY = kRY, class Epi>
+template<int KX, int WX, int WY, int STAGE, bool SINGLE = false, int RX = kRX, int RY = kRY, int BLOCKS = 0, class Epi>
 int launch_tile(const CUtensorMap& map, const TileArgs& a, const Epi& epi, cudaStream_t stream)
 {
-	auto kernel = conv_tile_kernel<KX, WX, WY, STAGE, Epi, SINGLE, RX, RY>;
+	auto kernel = [] {
+		if constexpr (BLOCKS > 0) return conv_tile_kernel_held<KX, WX, WY, STAGE, Epi, SINGLE, RX, RY, BLOCKS>;
+		else return conv_tile_kernel<KX, WX, WY, STAGE, Epi, SINGLE, RX, RY>;
+	}();
 	const int esize = (a.src_dtype == IANE_GB_U8 || a.src_dtype == IANE_GB_I8) ? 1 : 2;
 	const size_t smem = tile_smem_bytes<KX, WX, WY>(a.ky, a.kz, STAGE, esize);
 	IANE_GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),

@@ -187,6 +187,24 @@ def test_rl_volume_convolution_slabs(cuda):
         assert rel_err_bound(out[z0], ref, mag) <= FP32_TOL
 
 
+@pytest.mark.parametrize("shape,kernel,dtype", [
+    ((62, 187, 253), (3, 3, 5), np.float32), ((62, 190, 256), (3, 3, 7), np.float32),  # 744 tiles: five blocks per SM
+    ((20, 130, 333), (3, 5, 9), np.float32), ((20, 130, 336), (3, 5, 9), np.float32),  # 360 tiles, by copies and by TMA
+    ((1101, 1203), (5, 15), np.float32), ((1101, 1203), (7, 17), np.uint16),           # one plane, by copies
+    ((1101, 1216), (9, 9), np.uint8), ((9, 20, 21), (5, 9, 31), np.float32),           # narrow TMA; a tile wider than the image
+])
+def test_tile_staging(cuda, shape, kernel, dtype):
+    # n taps on positive data in FP32, one sum per kernel plane and those added up
+    rng = np.random.default_rng(sum(shape) + sum(kernel))
+    src = rng.random(shape, dtype=np.float32) + np.float32(0.01) if dtype is np.float32 else \
+        rng.integers(1, 200, shape).astype(dtype)
+    taps = rng.random(kernel, dtype=np.float32) + np.float32(0.1)
+    tol = (taps.size + 3) * 2.0 ** -24
+    for border in ("clamp", "zero", "mirror"):
+        ref = run_oracle(src, taps, np.float32, border)
+        assert float(np.max(np.abs(run_gpu(src, taps, np.float32, border) - ref) / ref)) <= tol, border
+
+
 @pytest.mark.parametrize("border", ["clamp", "zero", "mirror"])
 @pytest.mark.parametrize("shape,taps", [((40,), (7,)), ((33, 70), (7, 7)), ((512, 512), (7, 7)), ((9, 30, 75), (5, 3, 7)),
                                        ((20, 20, 20), (9, 9, 9)), ((3, 5, 4), (7, 9, 11)), ((70, 90), (21, 3)),
