@@ -304,20 +304,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity)
 	return done != 0;
 }
 
-// Whether the phase is complete, without waiting.
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity)
-{
-	uint32_t done;
-	asm volatile(
-		"{\n\t.reg .pred p;\n\t"
-		"mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-		"selp.u32 %0, 1, 0, p;\n\t}"
-		: "=r"(done)
-		: "r"(smem_addr(bar)), "r"(parity)
-		: "memory");
-	return done != 0;
-}
-
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar)
 {
 	asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
@@ -429,12 +415,6 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
 __device__ __forceinline__ void cp_async4(void* dst, const void* src, int src_bytes)
 {
 	asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(src_bytes)
-		: "memory");
-}
-// The same for 16 bytes (both addresses 16-byte aligned).
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, int src_bytes)
-{
-	asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(src_bytes)
 		: "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }

@@ -20,7 +20,6 @@
 #include "common.cuh"
 #include "kernels.h"
 
-
 namespace iane_gb {
 namespace {
 
@@ -384,7 +383,7 @@ int launch_conv_separable_fast(const DevView& src, const DevView* taps, const De
 	if (rows != IANE_GB_UNSUPPORTED) {
 		return rows;
 	}
-	// volumes of TMA-addressable rows, up to nine taps: separable_march.cu
+	// volumes of 16 or more along x and y, up to nine taps: separable_march.cu
 	if (src.rank > 2) {
 		const int march = launch_separable_march(src, taps, dst, border, r, stream);
 		if (march != IANE_GB_UNSUPPORTED) return march;

@@ -1,20 +1,25 @@
 // Separable FP32 convolution of 3-D f32 volumes (up to nine taps per axis): warps that march down z
 // on their own, as morphology_march.cu does.
 //
-// What bounds it: memory (8 B per voxel) and the FMA issue next to it. A block-wide kernel
-// that passes every plane through shared memory three times, with two block barriers
-// per pair of planes, waits at them: issue 59%, DRAM 41% of what they can. Here a lane owns 4
-// columns and 4 rows: it takes its rows and their neighbours from the warp's ring of input planes
-// (warp_ring.cuh, TMA two planes ahead), filters each row along x, the columns along y, and adds
-// the result to the 2 R unfinished outputs of every voxel along z, all in registers. The y and z
-// sums are packed two columns to an instruction, taps in pairs from shared memory.
+// What bounds it: memory (8 B per voxel) and the FMA issue next to it. A block-wide kernel that
+// passes every plane through shared memory three times, with two block barriers per pair of planes,
+// waits at them: issue 59%, DRAM 41% of what they can. Here a lane owns 4 columns and 4 rows: it takes
+// its rows and their neighbours from the warp's ring of input planes (warp_ring.cuh, two planes ahead
+// by TMA, or by 4-byte copies where TMA cannot address the rows), filters each row along x, the
+// columns along y, and adds the result to the 2 R unfinished outputs of every voxel along z, all in
+// registers. The y and z sums are packed two columns to an instruction, taps in pairs from shared
+// memory.
 // Mirror border, that kernel -> here: 512^3 3 taps 199 -> 176 us, 5 taps 255 -> 175 (90% of the
 // measured HBM rate), 7 taps 306 -> 246, 9 taps 401 -> 305; 256 x 256 x 64 7 taps 21.6 -> 18.6.
+// Rows of no multiple of 16 bytes: 253 x 181 x 60 3 taps 32 -> 14.5, 7 taps 63 -> 23, 511 x 401 x 301
+// 7 taps 451 -> 245.
 //
 // Rounding points are those of successive 1-D convolutions with an f32 intermediate; x and y sums
 // run from tap 0 up, the z sums from the oldest plane to the newest.
 #include "kernels.h"
 #include "warp_ring.cuh"
+
+#include <type_traits>
 
 namespace iane_gb {
 namespace {
@@ -33,8 +38,8 @@ struct MarchArgs {
 	int k[3];
 };
 
-template<int R, bool EDGE>
-__device__ __forceinline__ void filter_rows(const WarpRing<R>& ring, const float4* plane, const float (&tx)[2 * R + 1],
+template<int R, bool EDGE, class Ring>
+__device__ __forceinline__ void filter_rows(const Ring& ring, const float4* plane, const float (&tx)[2 * R + 1],
 	float2 (&h)[OUT + 2 * R][OUT / 2])
 {
 #pragma unroll
@@ -53,9 +58,9 @@ __device__ __forceinline__ void filter_rows(const WarpRing<R>& ring, const float
 	}
 }
 
-template<int R>
+template<int R, class Ring>
 __global__ void __launch_bounds__(32 * WARPS, R >= 3 ? 2 : R == 2 ? 3 : 4)
-	separable_march_kernel(const __grid_constant__ CUtensorMap map, const MarchArgs a)
+	separable_march_kernel(const __grid_constant__ typename Ring::Source source, const MarchArgs a)
 {
 	constexpr int K = 2 * R + 1;
 	constexpr int ROWS = OUT + 2 * R;
@@ -85,8 +90,8 @@ __global__ void __launch_bounds__(32 * WARPS, R >= 3 ? 2 : R == 2 ? 3 : 4)
 	}
 	__syncthreads();
 	if (y0 >= ny) return;
-	WarpRing<R> ring;
-	ring.begin(smem, WARPS, warp, &map, a.in, xw, y0, z0 - R, z1 + R);
+	Ring ring;
+	ring.begin(smem, WARPS, warp, &source, a.in, xw, y0, z0 - R, z1 + R);
 	const bool whole = x + OUT <= nx;
 	char* const column = a.dst + x * a.d_stride[0] + y0 * a.d_stride[1];
 
@@ -100,7 +105,7 @@ __global__ void __launch_bounds__(32 * WARPS, R >= 3 ? 2 : R == 2 ? 3 : 4)
 			for (int p = 0; p < PAIRS; ++p) pending[k][j][p] = make_float2(0.0f, 0.0f);
 
 	for (int z = z0 - R; z < z1 + R; ++z) {
-		const float4* plane = ring.plane(&map, a.in, z);
+		const float4* plane = ring.plane(&source, a.in, z);
 		float2 h[ROWS][PAIRS]; // every row filtered along x
 		if (ring.edge) {
 			filter_rows<R, true>(ring, plane, tx, h);
@@ -158,29 +163,39 @@ __global__ void __launch_bounds__(32 * WARPS, R >= 3 ? 2 : R == 2 ? 3 : 4)
 	}
 }
 
-template<int R>
-int launch(const DevView& s, MarchArgs a, cudaStream_t st)
+template<int R, class Ring>
+int launch_ring(const DevView& s, MarchArgs a, cudaStream_t st)
 {
-	constexpr size_t smem = WarpRing<R>::bytes(WARPS);
-	auto kernel = separable_march_kernel<R>;
+	constexpr size_t smem = Ring::bytes(WARPS);
+	auto kernel = separable_march_kernel<R, Ring>;
 	IANE_GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
 		"separable: set shared memory size");
-	CUtensorMap map{};
-	const int status = ring_map<R>(&map, s);
-	if (status) return status;
+	typename Ring::Source source{};
+	if constexpr (std::is_same_v<Ring, WarpRing<R>>) {
+		const int status = ring_map<R>(&source, s);
+		if (status) return status;
+	} else {
+		source = CopySource{s.ptr, s.stride[1], s.stride[2]};
+	}
 	const dim3 tiles((a.in.nx + kRingColumns - 1) / kRingColumns, (a.in.ny + OUT * WARPS - 1) / (OUT * WARPS));
 	a.zc = ring_chunk(static_cast<long long>(tiles.x) * tiles.y, a.in.nz, R,
 		static_cast<long long>(R >= 3 ? 2 : R == 2 ? 3 : 4) * device_sm_count());
-	kernel<<<dim3(tiles.x, tiles.y, (a.in.nz + a.zc - 1) / a.zc), dim3(32, WARPS), smem, st>>>(map, a);
+	kernel<<<dim3(tiles.x, tiles.y, (a.in.nz + a.zc - 1) / a.zc), dim3(32, WARPS), smem, st>>>(source, a);
 	IANE_GB_CUDA(cudaGetLastError(), "separable: launch");
 	return IANE_GB_OK;
+}
+
+template<int R>
+int launch(const DevView& s, const MarchArgs& a, cudaStream_t st)
+{
+	return ring_supported(s) ? launch_ring<R, WarpRing<R>>(s, a, st) : launch_ring<R, CopyRing<R>>(s, a, st);
 }
 
 }  // namespace
 
 int launch_separable_march(const DevView& src, const DevView* taps, const DevView& dst, int border, int r, cudaStream_t st)
 {
-	if (!ring_supported(src) || r > 4) return IANE_GB_UNSUPPORTED;
+	if (!ring_rows(src) || r > 4) return IANE_GB_UNSUPPORTED;
 	MarchArgs a{};
 	a.in = RingArgs{src.ext[0], src.ext[1], src.ext[2], border, device_status_ptr()};
 	if (!a.in.status) return IANE_GB_CUDA_ERROR;

@@ -25,8 +25,38 @@ struct RingArgs {
 	int* status;
 };
 
+// The four columns at `at` with R on either side.
+template<int R> __device__ __forceinline__ void ring_row(const float4* at, float (&w)[kRingOut + 2 * R])
+{
+	const float4 q = at[0];
+	w[R] = q.x;
+	w[R + 1] = q.y;
+	w[R + 2] = q.z;
+	w[R + 3] = q.w;
+	const float* beside = reinterpret_cast<const float*>(at);
+	if constexpr (R == 2) {
+		const float2 lo = *reinterpret_cast<const float2*>(beside - 2), hi = *reinterpret_cast<const float2*>(beside + 4);
+		w[0] = lo.x;
+		w[1] = lo.y;
+		w[6] = hi.x;
+		w[7] = hi.y;
+	} else if constexpr (R >= 3) {
+		const float4 lo = at[-1], hi = at[1];
+		const float l[4] = {lo.x, lo.y, lo.z, lo.w}, h[4] = {hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+		for (int j = 0; j < R; ++j) {
+			w[j] = l[4 - R + j];
+			w[R + kRingOut + j] = h[j];
+		}
+	} else {
+		w[0] = beside[-1];
+		w[R + kRingOut] = beside[kRingOut];
+	}
+}
+
 template<int R>
 struct WarpRing {
+	using Source = CUtensorMap;
 	static constexpr int ROWS = kRingOut + 2 * R;
 	static constexpr int PLANE = (ROWS * kRingGroups * 16 + 127) & ~127; // bytes; TMA writes to multiples of 128
 	static constexpr int RING = kRingStages * PLANE;
@@ -152,30 +182,7 @@ struct WarpRing {
 	template<bool EDGE> __device__ __forceinline__ void row(const float4* rows, int r, float (&w)[kRingOut + 2 * R]) const
 	{
 		const float4* at = rows + (EDGE ? static_cast<int>(from >> (4 * r) & 15u) : r) * kRingGroups + (threadIdx.x & 31) + 1;
-		const float4 q = at[0];
-		w[R] = q.x;
-		w[R + 1] = q.y;
-		w[R + 2] = q.z;
-		w[R + 3] = q.w;
-		const float* beside = reinterpret_cast<const float*>(at);
-		if constexpr (R == 2) {
-			const float2 lo = *reinterpret_cast<const float2*>(beside - 2), hi = *reinterpret_cast<const float2*>(beside + 4);
-			w[0] = lo.x;
-			w[1] = lo.y;
-			w[6] = hi.x;
-			w[7] = hi.y;
-		} else if constexpr (R >= 3) {
-			const float4 lo = at[-1], hi = at[1];
-			const float l[4] = {lo.x, lo.y, lo.z, lo.w}, h[4] = {hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-			for (int j = 0; j < R; ++j) {
-				w[j] = l[4 - R + j];
-				w[R + kRingOut + j] = h[j];
-			}
-		} else {
-			w[0] = beside[-1];
-			w[R + kRingOut] = beside[kRingOut];
-		}
+		ring_row<R>(at, w);
 		if constexpr (EDGE) {
 			// columns -1 - j and nx + j are columns j and nx - 1 - j under mirror
 #pragma unroll
@@ -188,10 +195,114 @@ struct WarpRing {
 	}
 };
 
-// Whether WarpRing can load from the view: TMA-addressable, 16 or more along x and y.
+// The same for rows that TMA cannot address: 4-byte cp.async, five per lane and row, from the columns and
+// rows that the border rule names, so that no edge is left to the reader. (253 x 181 x 60, 7 separable
+// taps, mirror: 23 us; the block-wide kernel, which maps every cell of a plane on its own, 63.)
+struct CopySource {
+	const char* src; // f32, contiguous along x; strides in bytes
+	long long s_row, s_plane;
+};
+
+template<int R>
+struct CopyRing {
+	using Source = CopySource;
+	static constexpr int ROWS = kRingOut + 2 * R;
+	static constexpr int PLANE = ROWS * kRingGroups * 16;
+	static constexpr int COPIES = (4 * kRingGroups + 31) / 32; // of a lane per row
+	static constexpr size_t bytes(int warps) { return static_cast<size_t>(warps) * (kRingStages * PLANE + 32 * COPIES * 4); }
+	static constexpr bool edge = false;
+
+	unsigned char* ring;
+	int* columns;            // the source column of each, or -1
+	unsigned long long from; // four bits per row, the row to read in its place
+	int y0, z1;
+	int slot;
+
+	__device__ __forceinline__ void begin(unsigned char* smem, int warps, int warp, const CopySource* s, const RingArgs& a, int x,
+		int y, int z, int z_end)
+	{
+		const int lane = threadIdx.x & 31;
+		ring = smem + warp * (kRingStages * PLANE);
+		columns = reinterpret_cast<int*>(smem + warps * (kRingStages * PLANE)) + warp * 32 * COPIES;
+		y0 = y;
+		z1 = z_end;
+		slot = 0;
+		from = 0;
+		for (int r = 0; r < ROWS; ++r) {
+			int yi = 0;
+			const int at = y0 - R + r;
+			// rows and columns that no stored output reads stay out
+			const int to = at < a.ny + R && map_coord(at, a.ny, a.border, yi) ? yi - (y0 - R) : 15; // among the warp's rows
+			from |= static_cast<unsigned long long>(to < 0 || to >= ROWS ? 15 : to) << (4 * r);
+		}
+		for (int k = lane; k < 32 * COPIES; k += 32) {
+			int xi = 0;
+			const int c = x - kRingOut + k;
+			columns[k] = c < a.nx + R && map_coord(c, a.nx, a.border, xi) ? xi : -1;
+		}
+		__syncwarp();
+		for (int k = 0; k < kRingStages - 1; ++k) copy(s, a, z + k, k);
+		prepare(a);
+	}
+
+	// The copy of plane z, if there is one, into slot `to`.
+	__device__ __forceinline__ void copy(const CopySource* s, const RingArgs& a, int z, int to)
+	{
+		const int lane = threadIdx.x & 31;
+		if (z < z1) {
+			int zi = 0;
+			const bool inside = map_coord(z, a.nz, a.border, zi);
+			const char* plane = s->src + zi * s->s_plane;
+			long long at[COPIES];
+			int bytes[COPIES];
+#pragma unroll
+			for (int k = 0; k < COPIES; ++k) {
+				const int xi = columns[32 * k + lane];
+				at[k] = 4LL * max(xi, 0);
+				bytes[k] = inside && xi >= 0 ? 4 : 0;
+			}
+			float* cells = reinterpret_cast<float*>(ring + to * PLANE) + lane;
+#pragma unroll 2
+			for (int r = 0; r < ROWS; ++r, cells += 4 * kRingGroups) {
+				const int f = static_cast<int>(from >> (4 * r) & 15u);
+				const char* row = plane + (f < ROWS ? y0 - R + f : 0) * s->s_row;
+#pragma unroll
+				for (int k = 0; k < COPIES; ++k) {
+					if (32 * k + lane < 4 * kRingGroups) cp_async4(cells + 32 * k, row + at[k], f < ROWS ? bytes[k] : 0);
+				}
+			}
+		}
+		cp_async_commit(); // empty past the end, so that prepare() can count
+	}
+
+	__device__ __forceinline__ const float4* plane(const CopySource* s, const RingArgs& a, int z)
+	{
+		__syncwarp();
+		copy(s, a, z + kRingStages - 1, slot == 0 ? kRingStages - 1 : slot - 1);
+		const float4* rows = reinterpret_cast<const float4*>(ring + slot * PLANE);
+		if (++slot == kRingStages) slot = 0;
+		return rows;
+	}
+
+	// plane() brings the warp together.
+	__device__ __forceinline__ void prepare(const RingArgs&) { cp_async_wait<kRingStages - 2>(); }
+
+	template<bool EDGE> __device__ __forceinline__ void row(const float4* rows, int r, float (&w)[kRingOut + 2 * R]) const
+	{
+		ring_row<R>(rows + r * kRingGroups + (threadIdx.x & 31) + 1, w);
+	}
+};
+
+// Whether CopyRing can load from the view: f32 contiguous along x, 16 or more along x and y.
+inline bool ring_rows(const DevView& s)
+{
+	return s.dtype == IANE_GB_F32 && s.stride[0] == 4 && s.ext[0] >= 16 && s.ext[1] >= 16;
+}
+
+// and WarpRing: TMA-addressable
 inline bool ring_supported(const DevView& s)
 {
-	return s.dtype == IANE_GB_F32 && rows_aligned16(s) && s.stride[1] >= 4LL * s.ext[0] && s.ext[0] >= 16 && s.ext[1] >= 16 &&
+	return ring_rows(s) && rows_aligned16(s) && s.stride[1] >= 4LL * s.ext[0] &&
 		(s.ext[2] <= 1 || s.stride[2] >= s.stride[1] * s.ext[1]);
 }
 
