@@ -91,9 +91,36 @@ __global__ void wiener_make_filter(float2* h, long long nc, double noise)
 // where packed rows are aligned for it; blocks stride over the rows. What bounds them is memory
 // (5 B per u8 pixel); with one element per thread and step they spent their time on the two
 // 64-bit index divisions of each. 2560 x 1920 u8, ncu, cold: load 25 us and store 26 us then,
-// 9 and 11 now.
+// 9 and 11 now. Narrow rows and small images leave most of a block without elements, and its
+// latency shows: below, one element per thread (331 x 544 u8, a whole run: 29.6 us so, 31.9 by
+// rows; 129 x 2600 47.6 and 52; 1200 x 700 the other way, 53 and 48).
 constexpr int kGroups = 4;
 constexpr int kRun = 256 * 4 * kGroups;
+
+bool by_element(const DevView& v)
+{
+	const long long n = element_count(v);
+	return (n < (1LL << 19) || v.ext[0] < 1024) && n < (1LL << 31);
+}
+
+// Element i of the view in packed order.
+__device__ __forceinline__ char* packed_element(const DevView& v, uint32_t i)
+{
+	const uint32_t row = i / v.ext[0], z = row / v.ext[1];
+	return v.ptr + (i - row * v.ext[0]) * v.stride[0] + (row - z * v.ext[1]) * v.stride[1] + z * v.stride[2];
+}
+
+__global__ void __launch_bounds__(256) wiener_load_element(DevView src, float* out, uint32_t n)
+{
+	const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+	if (i < n) out[i] = load_as_float(packed_element(src, i), src.dtype);
+}
+
+__global__ void __launch_bounds__(256) wiener_store_element(const float* __restrict__ real, float scale, DevView dst, uint32_t n)
+{
+	const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+	if (i < n) store_converted_f32(packed_element(dst, i), dst.dtype, real[i] * scale);
+}
 
 dim3 row_grid(const DevView& v)
 {
@@ -366,7 +393,12 @@ int iane_gb_wiener_run(iane_gb_wiener_plan* plan, const iane_gb_view* observed, 
 	cufftComplex* spec = reinterpret_cast<cufftComplex*>(base);
 	base += align_up(static_cast<size_t>(plan->nc) * sizeof(float2));
 	void* work = base;
-	wiener_load<<<row_grid(s), 256, 0, st>>>(s, real);
+	const uint32_t n = static_cast<uint32_t>(plan->n), blocks = static_cast<uint32_t>((plan->n + 255) / 256);
+	if (by_element(s)) {
+		wiener_load_element<<<blocks, 256, 0, st>>>(s, real, n);
+	} else {
+		wiener_load<<<row_grid(s), 256, 0, st>>>(s, real);
+	}
 	if (cufftSetStream(plan->r2c, st) != CUFFT_SUCCESS || cufftSetStream(plan->c2r, st) != CUFFT_SUCCESS ||
 	    cufftSetWorkArea(plan->r2c, work) != CUFFT_SUCCESS || cufftSetWorkArea(plan->c2r, work) != CUFFT_SUCCESS ||
 	    cufftExecR2C(plan->r2c, real, spec) != CUFFT_SUCCESS) {
@@ -378,7 +410,11 @@ int iane_gb_wiener_run(iane_gb_wiener_plan* plan, const iane_gb_view* observed, 
 	}
 	// main.cu:74: scale = 1 / (w h) in double, rounded to float
 	const float scale = static_cast<float>(1.0 / static_cast<double>(plan->n));
-	wiener_store<<<row_grid(d), 256, 0, st>>>(real, scale, d);
+	if (by_element(d)) {
+		wiener_store_element<<<blocks, 256, 0, st>>>(real, scale, d, n);
+	} else {
+		wiener_store<<<row_grid(d), 256, 0, st>>>(real, scale, d);
+	}
 	IANE_GB_CUDA(cudaGetLastError(), "wiener run: kernels");
 	return IANE_GB_OK;
 }

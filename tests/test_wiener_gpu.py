@@ -98,7 +98,7 @@ def test_wiener_errors(cuda):
     w.close()
 
 
-@pytest.mark.parametrize("shape", [(7, 5), (3, 1025), (2, 4099), (2, 3, 4096)], ids=str)
+@pytest.mark.parametrize("shape", [(7, 5), (3, 1025), (2, 4099), (2, 3, 4096), (520, 1025), (130, 4099), (2, 65, 4096)], ids=str)
 @pytest.mark.parametrize("dtype", [np.uint8, np.float32], ids=lambda d: np.dtype(d).name)
 def test_aligned_and_unaligned_rows_give_the_same_bits(cuda, shape, dtype):
     # packed images take word loads and stores where rows allow; crops that start one element into
