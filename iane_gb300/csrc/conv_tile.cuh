@@ -40,7 +40,11 @@
 
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace iane_gb {
+
+struct EpiStoreF32;
 
 constexpr int kRX = 8;
 constexpr int kRY = 4;
@@ -564,7 +568,12 @@ __device__ __forceinline__ void conv_tile_block(const CUtensorMap& tmap, const T
 		}
 	}
 	uint32_t phases = 0;
-	const int x0 = blockIdx.x * 32 * WX, y0 = blockIdx.y * 32 * WY;
+	// Planes on their own: the bottom row of tiles first, as edge tiles take longer and the last wave is
+	// better without them (2560 x 1920 u8 9 x 9 clamp 30.5 -> 29.3 us). Volumes gain nothing, and the
+	// Richardson-Lucy epilogues' partial sums keep their order.
+	constexpr bool ROTATE = SINGLE && std::is_same_v<Epi, EpiStoreF32>;
+	const unsigned row = !ROTATE ? blockIdx.y : blockIdx.y == 0 ? gridDim.y - 1 : blockIdx.y - 1;
+	const int x0 = blockIdx.x * 32 * WX, y0 = row * 32 * WY;
 	float acc[RY][RX];
 	conv_tile_sums<KX, WX, WY, STAGE, SINGLE, RX, RY, SINGLE>(&tmap, a, x0, y0, blockIdx.z, phases,
 		tile_barriers<KX, WX, WY>(a.ky, a.kz), acc);
