@@ -2,6 +2,7 @@
 #pragma once
 
 #include "../../include/iane_gb/capi.h"
+#include "counters.h"
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -345,17 +346,18 @@ __device__ __forceinline__ void fence_proxy_async_global()
 	asm volatile("fence.proxy.async.global;" ::: "memory");
 }
 
-// Bounded wait until *word >= need. False if the run was aborted or the wait gave up after
-// `limit_ns` of global time (which it records in the status word and turns into an abort).
+// Bounded wait until *word has reached need (counter_reached). False if the run was aborted or the
+// wait gave up after `limit_ns` of global time (which it records in the status word and turns into
+// an abort).
 __device__ __forceinline__ bool wait_counter(const unsigned int* word, unsigned int need, int* abort, int* status,
 	uint64_t limit_ns = 2000000000ull)
 {
-	if (load_acquire(word) >= need) {
+	if (counter_reached(load_acquire(word), need)) {
 		return true;
 	}
 	const uint64_t t0 = global_ns();
 	for (uint32_t i = 1; i < (1u << 26); ++i) {
-		if (load_acquire(word) >= need) {
+		if (counter_reached(load_acquire(word), need)) {
 			return true;
 		}
 		if (load_volatile(abort)) {

@@ -10,8 +10,8 @@
 // RL's only dependency is per image: a phase of an image reads (with a halo) what the image's
 // previous phase wrote and overwrites what it read, so an item of phase p waits until all
 // tiles of its image's phase p - 1 are done -- a per-image completion counter that reaches
-// p * 4 * tiles, counted by warps -- instead of a grid-wide drain between passes. Images of the
-// next phase start as soon as their own previous pass is complete.
+// p * 4 * tiles (modulo 2^32), counted by warps -- instead of a grid-wide drain between passes.
+// Images of the next phase start as soon as their own previous pass is complete.
 //
 // Progress: an item waits only for items earlier in the queue, which were handed to CTAs that
 // are running, so the earliest unfinished item can always proceed. Every wait is bounded (two

@@ -121,7 +121,7 @@ __device__ __forceinline__ void take_tile(const FeedArgs& a, const BatchQueues& 
 // Completions of the image's previous phases that the tile in hand needs (four warps a tile).
 __device__ __forceinline__ unsigned int tile_need(const BatchShared& sh)
 {
-	return static_cast<unsigned int>(sh.phase) * 4u * static_cast<unsigned int>(sh.item.image_tiles);
+	return batch_need(sh.phase, sh.item.image_tiles);
 }
 
 // Thread 0, the buffers being free and the image's previous phase complete: hand on the tile.
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(128, 4) batch_persistent_kernel(const BatchIma
 		__syncthreads(); // tile and taps have been read
 		bool waiting = false;
 		if (t == 0) {
-			waiting = sh->phase > 0 && load_acquire(sync.done + sh->item.image) < tile_need(*sh);
+			waiting = sh->phase > 0 && !counter_reached(load_acquire(sync.done + sh->item.image), tile_need(*sh));
 			if (!waiting) issue_tile(feed);
 		}
 		const int xo = wx + kRX * (lane & 3), yo = wy + kRY * (lane >> 2);
