@@ -271,10 +271,10 @@ __global__ void __launch_bounds__(THREADS) cnn_tc_conv_kernel(const __grid_const
 			const bool valid = (r & 15) >= 1 && (r & 15) <= OUT_X && x < a.w && y < a.h;
 			const long long v0 = z0 * plane + static_cast<long long>(y) * a.w + x;
 			wait(&ready[set], (i / 2) & 1);
-			__syncwarp(); // tcgen05.ld is warp-collective
-			tc::fence_after_sync();
 #pragma unroll 1
 			for (int q = 0; q < BZ * (N / 16); ++q) {
+				__syncwarp(); // tcgen05.ld is warp-collective: lanes come from the wait or from `continue`
+				tc::fence_after_sync();
 				const int zb = q / (N / 16), j = q % (N / 16);
 				const long long v = zb ? v0 + plane : v0;
 				float d0[16], d1[16], d2[16];
