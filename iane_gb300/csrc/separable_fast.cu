@@ -271,10 +271,11 @@ __global__ void __launch_bounds__(kFThreads) separable_fast_kernel(const __grid_
 	};
 
 	if constexpr (!Z) {
+		const float tz = tpair[16 + R].x; // the single tap along z of a volume's one plane, or 1
 		for (int p = 0; p < nplanes; ++p) {
 			float2 c0, c1;
 			filter_plane(p, c0, c1);
-			store(0, y0_of(p), c0, c1);
+			store(0, y0_of(p), make_float2(c0.x * tz, c0.y * tz), make_float2(c1.x * tz, c1.y * tz));
 		}
 	} else {
 		for (int p = 0; p < nplanes; ++p) {
@@ -324,7 +325,7 @@ int launch_radius(const DevView& src, const DevView* taps, const DevView& dst, i
 		a.tap_stride[axis] = taps[axis].stride[0];
 		a.k[axis] = taps[axis].ext[0];
 	}
-	const bool z3 = src.rank > 2; // also of one plane: its tap along z counts
+	const bool z3 = !separable_2d(src, taps);
 	// TMA wants positive, 16-byte multiple pitches that do not make rows or planes overlap.
 	a.use_tma = (rows_aligned16(src) && (src.ext[1] <= 1 || src.stride[1] >= 4LL * src.ext[0]) &&
 		(src.ext[2] <= 1 || (src.stride[2] > 0 && src.stride[2] >= (src.ext[1] > 1 ? src.stride[1] : 4LL * src.ext[0]) *
@@ -384,7 +385,7 @@ int launch_conv_separable_fast(const DevView& src, const DevView* taps, const De
 		return rows;
 	}
 	// volumes of 16 or more along x and y, up to nine taps: separable_march.cu
-	if (src.rank > 2) {
+	if (!separable_2d(src, taps)) {
 		const int march = launch_separable_march(src, taps, dst, border, r, stream);
 		if (march != IANE_GB_UNSUPPORTED) return march;
 	}

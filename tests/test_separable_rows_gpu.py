@@ -75,3 +75,22 @@ def test_interior_equals_the_tiled_kernel_bit_for_bit(cuda):
     got = to_host(big)[y0 + r:y0 + n - r, x0 + r:x0 + n - r]
     want = to_host(crop)[r:n - r, r:n - r]
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("border", ["clamp", "mirror", "zero"])
+@pytest.mark.parametrize("shape,kx,ky", [((64, 70), 3, 3), ((33, 65), 9, 5), ((700, 901), 7, 7), ((2048, 2080), 5, 9)])
+def test_one_plane_of_a_volume_takes_the_2d_kernels(cuda, shape, kx, ky, border):
+    # under a single tap along z: the image's result times the tap, rounded once, and an infinite
+    # pixel reaches what it reaches in the image
+    rng = np.random.default_rng(sum(shape) + kx)
+    src = rng.random(shape, dtype=np.float32) - np.float32(0.3)
+    src[shape[0] // 2, shape[1] // 3] = np.inf
+    src[0, 0] = -np.inf
+    t = [to_gpu(taps(kx, kx / 4)), to_gpu(taps(ky, ky / 5))]
+    image = empty_like_np(shape, np.float32)
+    iane_gb300.convolve_separable(to_gpu(src), t, image, border)
+    want = to_host(image)
+    for tap in (1.0, 0.7, -3.0):
+        volume = empty_like_np((1, *shape), np.float32)
+        iane_gb300.convolve_separable(to_gpu(src[None]), t + [to_gpu(np.float32([tap]))], volume, border)
+        assert np.array_equal(to_host(volume)[0], want * np.float32(tap), equal_nan=True), tap
