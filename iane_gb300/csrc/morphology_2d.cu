@@ -18,6 +18,7 @@
 // (floor 5.8); 4096 x 4096 u8 83 and 13.2.
 #include "common.cuh"
 #include "kernels.h"
+#include "plane_lanes.h"
 
 #include <limits>
 #include <type_traits>
@@ -70,15 +71,15 @@ template<int N> __device__ __forceinline__ uint32_t map_run(int first, int n, in
 
 // R: the largest radius of this instantiation (rx, ry <= R).
 template<class T, bool DILATE, int R>
-__global__ void __launch_bounds__(128) morph_plane_int_kernel(const Plane2D a)
+__global__ void __launch_bounds__(kPlaneThreads) morph_plane_int_kernel(const Plane2D a)
 {
 	using P = Pairs<T, DILATE>;
 	constexpr int PX = 8;
 	constexpr int PAD = (R + 1) & ~1;                 // elements before the first, a whole number of pairs
 	constexpr int NP = (PX + 2 * PAD) / 2;            // pairs of a row
 	constexpr int WORDS = (PX + 2 * PAD) * sizeof(T) / 4; // 32-bit words of a row
-	const int x0 = (blockIdx.x * 32 + threadIdx.x) * PX;
-	const int y0 = (blockIdx.y * 4 + threadIdx.y) * ROWS;
+	const int x0 = (blockIdx.x * blockDim.x + threadIdx.x) * PX;
+	const int y0 = (blockIdx.y * blockDim.y + threadIdx.y) * ROWS;
 	if (x0 >= a.nx || y0 >= a.ny) return;
 	const char* src = a.src + static_cast<long long>(blockIdx.z) * a.s_plane;
 	// whole words around the window stay inside the row (up to 3 bytes more on either side)
@@ -207,13 +208,13 @@ template<bool DILATE> __device__ __forceinline__ void take_f32(float v, float& r
 }
 
 template<bool DILATE, int R>
-__global__ void __launch_bounds__(128) morph_plane_f32_kernel(const Plane2D a)
+__global__ void __launch_bounds__(kPlaneThreads) morph_plane_f32_kernel(const Plane2D a)
 {
 	constexpr int PX = 4, ROWS = 4;
 	constexpr int N = PX + 2 * R;
 	const float start = DILATE ? -std::numeric_limits<float>::infinity() : std::numeric_limits<float>::infinity();
-	const int x0 = (blockIdx.x * 32 + threadIdx.x) * PX;
-	const int y0 = (blockIdx.y * 4 + threadIdx.y) * ROWS;
+	const int x0 = (blockIdx.x * blockDim.x + threadIdx.x) * PX;
+	const int y0 = (blockIdx.y * blockDim.y + threadIdx.y) * ROWS;
 	if (x0 >= a.nx || y0 >= a.ny) return;
 	const char* src = a.src + static_cast<long long>(blockIdx.z) * a.s_plane;
 	const bool inside = x0 - 4 >= 0 && x0 + PX + 4 <= a.nx;
@@ -291,40 +292,50 @@ bool rows16(const DevView& v)
 		(v.ext[2] <= 1 || v.stride[2] % 16 == 0);
 }
 
-template<class T, bool DILATE, int R>
-void launch_radius(const Plane2D& a, int planes, cudaStream_t st)
+struct Shape {
+	dim3 block, grid;
+};
+
+Shape shape_of(const Plane2D& a, int planes, bool f32, int r)
 {
-	constexpr int px = std::is_same_v<T, float> ? 4 : 8, rows = std::is_same_v<T, float> ? 4 : ROWS;
-	const dim3 grid((a.nx + 32 * px - 1) / (32 * px), (a.ny + 4 * rows - 1) / (4 * rows), planes);
+	const int px = f32 ? 4 : 8, rows = f32 ? 4 : ROWS;
+	const int lanes = plane_lanes(a.nx, a.ny, px, rows, a.src16 != 0, r);
+	const int w = lanes * px, h = kPlaneThreads / lanes * rows;
+	return Shape{dim3(lanes, kPlaneThreads / lanes), dim3((a.nx + w - 1) / w, (a.ny + h - 1) / h, planes)};
+}
+
+template<class T, bool DILATE, int R>
+void launch_radius(const Plane2D& a, const Shape& s, cudaStream_t st)
+{
 	if constexpr (std::is_same_v<T, float>) {
-		morph_plane_f32_kernel<DILATE, R><<<grid, dim3(32, 4), 0, st>>>(a);
+		morph_plane_f32_kernel<DILATE, R><<<s.grid, s.block, 0, st>>>(a);
 	} else {
-		morph_plane_int_kernel<T, DILATE, R><<<grid, dim3(32, 4), 0, st>>>(a);
+		morph_plane_int_kernel<T, DILATE, R><<<s.grid, s.block, 0, st>>>(a);
 	}
 }
 
 template<class T, bool DILATE>
-void launch_op(const Plane2D& a, int planes, cudaStream_t st)
+void launch_op(const Plane2D& a, const Shape& s, cudaStream_t st)
 {
 	const int r = a.rx > a.ry ? a.rx : a.ry;
 	if (r <= 1) {
-		launch_radius<T, DILATE, 1>(a, planes, st);
+		launch_radius<T, DILATE, 1>(a, s, st);
 	} else if (r == 2) {
-		launch_radius<T, DILATE, 2>(a, planes, st);
+		launch_radius<T, DILATE, 2>(a, s, st);
 	} else if (r == 3) {
-		launch_radius<T, DILATE, 3>(a, planes, st);
+		launch_radius<T, DILATE, 3>(a, s, st);
 	} else {
-		launch_radius<T, DILATE, 4>(a, planes, st);
+		launch_radius<T, DILATE, 4>(a, s, st);
 	}
 }
 
 template<class T>
-void launch_typed(const Plane2D& a, int planes, bool dilate, cudaStream_t st)
+void launch_typed(const Plane2D& a, const Shape& s, bool dilate, cudaStream_t st)
 {
 	if (dilate) {
-		launch_op<T, true>(a, planes, st);
+		launch_op<T, true>(a, s, st);
 	} else {
-		launch_op<T, false>(a, planes, st);
+		launch_op<T, false>(a, s, st);
 	}
 }
 
@@ -353,19 +364,27 @@ int launch_morph_planes(const DevView& s, const DevView& d, const int* r, bool d
 	// Radii of 3 and 4 stay on the tiled kernel where the longer threads do not pay: images too
 	// small for a block per SM (300 x 256 u8, 9 x 9: 4.6 us tiled, 6.0 here; 1533 x 1001: 11.5 and
 	// 7.9), and f32 rows that take a load per sample (9 x 9 on 40 planes of 513 x 300: 51 tiled, 64
-	// here; 16-byte aligned rows, 2560 x 1920: 37 and 34).
+	// here; 16-byte aligned rows, 2560 x 1920: 37 and 34). So do f32 windows nine wide on narrow rows or
+	// less than nine tall, whose chains of compares along x the other threads of a row do not hide,
+	// and windows seven wide and up to three tall on the narrowest (8e6 elements, zero border: 9 x 9 on 200
+	// columns 64 us tiled, 68 here, on 512 59 and 57; 9 x 3 on 2560 42 and 47; 1 x 9 on 4000 43 and 44;
+	// 7 x 1 on 60 42 and 46).
 	const bool f32 = s.dtype == IANE_GB_F32;
-	if (r[0] > 2 || r[1] > 2) {
-		const long long blocks = static_cast<long long>((a.nx + (f32 ? 127 : 255)) / (f32 ? 128 : 256)) *
-			((a.ny + (f32 ? 15 : 31)) / (f32 ? 16 : 32)) * s.ext[2];
+	const int most = r[0] > r[1] ? r[0] : r[1];
+	const Shape shape = shape_of(a, s.ext[2], f32, most);
+	if (most > 2) {
+		const long long blocks = static_cast<long long>(shape.grid.x) * shape.grid.y * shape.grid.z;
 		if (blocks < device_sm_count() || (f32 && !a.src16)) return IANE_GB_UNSUPPORTED;
+		if (f32 && (most == 4 ? r[0] == 0 || r[1] != 4 || a.nx < 512 : r[0] == 3 && r[1] <= 1 && a.nx < 100)) {
+			return IANE_GB_UNSUPPORTED;
+		}
 	}
 	switch (s.dtype) {
-	case IANE_GB_U8: launch_typed<uint8_t>(a, s.ext[2], dilate, st); break;
-	case IANE_GB_I8: launch_typed<int8_t>(a, s.ext[2], dilate, st); break;
-	case IANE_GB_U16: launch_typed<uint16_t>(a, s.ext[2], dilate, st); break;
-	case IANE_GB_I16: launch_typed<int16_t>(a, s.ext[2], dilate, st); break;
-	case IANE_GB_F32: launch_typed<float>(a, s.ext[2], dilate, st); break;
+	case IANE_GB_U8: launch_typed<uint8_t>(a, shape, dilate, st); break;
+	case IANE_GB_I8: launch_typed<int8_t>(a, shape, dilate, st); break;
+	case IANE_GB_U16: launch_typed<uint16_t>(a, shape, dilate, st); break;
+	case IANE_GB_I16: launch_typed<int16_t>(a, shape, dilate, st); break;
+	case IANE_GB_F32: launch_typed<float>(a, shape, dilate, st); break;
 	default: return IANE_GB_UNSUPPORTED;
 	}
 	IANE_GB_CUDA(cudaGetLastError(), "morphology: launch");

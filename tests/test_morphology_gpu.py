@@ -239,3 +239,25 @@ def test_volumes_of_aligned_rows(cuda, shape, radius):
                 got = to_host(out)
                 assert np.ascontiguousarray(got[..., 1:]).tobytes() == ref.tobytes(), (op, border, "crop")
                 assert not got[..., 0].any()
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.int16, np.float32], ids=lambda d: np.dtype(d).name)
+@pytest.mark.parametrize("shape,radius", [
+    ((600, 3), (2, 1)), ((2500, 12), (3, 3)),     # blocks of one and of two to four threads side by side
+    ((1500, 60), (1, 3)), ((1500, 100), (4, 4)),  # of eight; as narrow as a rule's limit
+    ((2000, 300), (1, 2)), ((900, 516), (4, 4)),  # of eight and sixteen beyond whole blocks
+    ((70, 4100), (2, 2)),                         # an image lower than the tallest blocks
+])
+def test_planes_of_narrow_images(cuda, dtype, shape, radius):
+    rng = np.random.default_rng(zlib.crc32(repr((np.dtype(dtype).name, shape, radius)).encode()))
+    if dtype == np.float32:
+        src = rng.standard_normal(shape).astype(dtype)
+        for value in (np.nan, 0.0, -0.0, -np.inf):
+            src[rng.random(shape) < 0.05] = value
+    else:
+        info = np.iinfo(dtype)
+        src = rng.integers(info.min, info.max, shape, dtype=dtype, endpoint=True)
+    for op, border in (("erode", "clamp"), ("dilate", "zero"), ("erode", "mirror")):
+        ref = np.zeros_like(src)
+        oracle.morphology(src, ref, radius, op, border)
+        assert run_gpu(src, radius, op, border).tobytes() == ref.tobytes(), (op, border)
