@@ -9,6 +9,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "ring_chunk.h"
 
 namespace iane_gb {
 
@@ -310,26 +311,6 @@ template<int R> int ring_map(CUtensorMap* map, const DevView& s)
 {
 	return encode_tensor_map_f32(map, s.ptr, s.ext[0], s.ext[1], s.ext[2], s.stride[1],
 		s.ext[2] > 1 ? s.stride[2] : s.stride[1] * s.ext[1], 4 * kRingGroups, WarpRing<R>::ROWS);
-}
-
-// Output planes per block: every chunk reads 2 r more, so as long as fills whole waves of `slots`
-// resident blocks; `columns` blocks side by side.
-inline int ring_chunk(long long columns, int nz, int r, long long slots)
-{
-	double best = -1.0;
-	int best_zc = nz;
-	for (int chunks = 1; chunks <= nz; ++chunks) {
-		const int zc = (nz + chunks - 1) / chunks;
-		const long long blocks = columns * ((nz + zc - 1) / zc);
-		const double waves = static_cast<double>(blocks) / static_cast<double>(slots);
-		const double score = waves / static_cast<double>((blocks + slots - 1) / slots) * zc / (zc + 2.0 * r);
-		if (score > best + 1e-9) {
-			best = score;
-			best_zc = zc;
-		}
-		if (waves > 8.0) break;
-	}
-	return best_zc;
 }
 
 }  // namespace iane_gb
