@@ -100,14 +100,14 @@ __device__ __forceinline__ void four_windows(const float (&v)[OUT + 2 * R], floa
 
 // The x windows of a plane's rows. Returns whether one of the samples is -0 (the lowest integer by
 // its bits) in any lane.
-template<bool DILATE, bool FAST, int R, bool EDGE>
-__device__ __forceinline__ bool x_windows(const WarpRing<R>& ring, const float4* plane, float (&h)[OUT + 2 * R][OUT])
+template<bool DILATE, bool FAST, int R, bool EDGE, class Ring>
+__device__ __forceinline__ bool x_windows(const Ring& ring, const float4* plane, float (&h)[OUT + 2 * R][OUT])
 {
 	int low = 0;
 #pragma unroll
 	for (int r = 0; r < OUT + 2 * R; ++r) {
 		float w[OUT + 2 * R];
-		ring.template row<EDGE>(plane, r, w);
+		ring.template read<EDGE>(plane, r, w);
 #pragma unroll
 		for (int i = 0; i < OUT + 2 * R; ++i) low = min(low, __float_as_int(w[i]));
 		four_windows<DILATE, FAST, R>(w, h[r]);
@@ -150,22 +150,22 @@ __device__ __forceinline__ void z_windows(float (&pending)[2 * R][OUT][OUT], flo
 	}
 }
 
-template<bool DILATE, int R>
+template<bool DILATE, int R, int LANES>
 __global__ void __launch_bounds__(32 * WARPS, R == 3 ? 2 : R == 2 ? 3 : 4)
 	morph_march_kernel(const __grid_constant__ CUtensorMap map, const MarchArgs a)
 {
+	using Ring = WarpRing<R, LANES>;
 	constexpr int ROWS = OUT + 2 * R;
 	extern __shared__ __align__(128) unsigned char smem[];
-	const int lane = threadIdx.x, warp = threadIdx.y;
+	const int warp = threadIdx.y, warps = LANES == 32 ? WARPS : blockDim.y;
 	const int nx = a.in.nx, ny = a.in.ny;
-	const int xw = blockIdx.x * kRingColumns; // the warp's first column
-	const int x = xw + OUT * lane;
-	const int y0 = (blockIdx.y * WARPS + warp) * OUT;
+	const int xw = blockIdx.x * Ring::COLUMNS, yw = (blockIdx.y * warps + warp) * Ring::OUT_ROWS; // the warp's first
+	const int x = xw + Ring::column(), y0 = yw + Ring::row();
 	const int z0 = blockIdx.z * a.zc, z1 = min(a.in.nz, z0 + a.zc);
-	if (y0 >= ny) return;
+	if (yw >= ny) return;
 	const bool whole = x + OUT <= nx;
-	WarpRing<R> ring;
-	ring.begin(smem, WARPS, warp, &map, a.in, xw, y0, z0 - R, z1 + R);
+	Ring ring;
+	ring.begin(smem, warps, warp, &map, a.in, xw, yw, z0 - R, z1 + R);
 
 	// unfinished outputs: pending[k] has seen its first 2 R - k planes
 	float pending[2 * R][OUT][OUT];
@@ -219,22 +219,30 @@ __global__ void __launch_bounds__(32 * WARPS, R == 3 ? 2 : R == 2 ? 3 : 4)
 	}
 }
 
-template<bool DILATE, int R>
-int launch(const DevView& s, MarchArgs a, cudaStream_t st)
+template<bool DILATE, int R, int LANES>
+int launch_lanes(const DevView& s, MarchArgs a, cudaStream_t st)
 {
-	constexpr size_t smem = WarpRing<R>::bytes(WARPS);
-	auto kernel = morph_march_kernel<DILATE, R>;
+	using Ring = WarpRing<R, LANES>;
+	const int warps = ring_warps<Ring>(a.in, WARPS);
+	const size_t smem = Ring::bytes(warps);
+	auto kernel = morph_march_kernel<DILATE, R, LANES>;
 	IANE_GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
 		"morphology: set shared memory size");
 	CUtensorMap map{};
-	const int status = ring_map<R>(&map, s);
+	const int status = ring_map<R, LANES>(&map, s);
 	if (status) return status;
-	const dim3 tiles((a.in.nx + kRingColumns - 1) / kRingColumns, (a.in.ny + OUT * WARPS - 1) / (OUT * WARPS));
+	const dim3 tiles = ring_tiles<Ring>(a.in, warps);
 	a.zc = ring_chunk(static_cast<long long>(tiles.x) * tiles.y, a.in.nz, R,
-		static_cast<long long>(R == 3 ? 2 : R == 2 ? 3 : 4) * device_sm_count());
-	kernel<<<dim3(tiles.x, tiles.y, (a.in.nz + a.zc - 1) / a.zc), dim3(32, WARPS), smem, st>>>(map, a);
+		static_cast<long long>((R == 3 ? 2 : R == 2 ? 3 : 4) * WARPS / warps) * device_sm_count());
+	kernel<<<dim3(tiles.x, tiles.y, (a.in.nz + a.zc - 1) / a.zc), dim3(32, warps), smem, st>>>(map, a);
 	IANE_GB_CUDA(cudaGetLastError(), "morphology: launch");
 	return IANE_GB_OK;
+}
+
+template<bool DILATE, int R>
+int launch(const DevView& s, const MarchArgs& a, cudaStream_t st)
+{
+	return ring_narrow(a.in.nx, 1 << 30) ? launch_lanes<DILATE, R, 16>(s, a, st) : launch_lanes<DILATE, R, 32>(s, a, st);
 }
 
 template<bool DILATE>

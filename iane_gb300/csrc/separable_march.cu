@@ -45,7 +45,7 @@ __device__ __forceinline__ void filter_rows(const Ring& ring, const float4* plan
 #pragma unroll
 	for (int r = 0; r < OUT + 2 * R; ++r) {
 		float w[OUT + 2 * R], o[OUT];
-		ring.template row<EDGE>(plane, r, w);
+		ring.template read<EDGE>(plane, r, w);
 #pragma unroll
 		for (int i = 0; i < OUT; ++i) {
 			float s = 0.0f;
@@ -67,11 +67,10 @@ __global__ void __launch_bounds__(32 * WARPS, R >= 3 ? 2 : R == 2 ? 3 : 4)
 	constexpr int PAIRS = OUT / 2;
 	extern __shared__ __align__(128) unsigned char smem[];
 	__shared__ float2 taps[2][K]; // (t, t) of axes 1 and 2
-	const int lane = threadIdx.x, warp = threadIdx.y;
+	const int lane = threadIdx.x, warp = threadIdx.y, warps = Ring::LANES == 32 ? WARPS : blockDim.y;
 	const int nx = a.in.nx, ny = a.in.ny;
-	const int xw = blockIdx.x * kRingColumns;
-	const int x = xw + OUT * lane;
-	const int y0 = (blockIdx.y * WARPS + warp) * OUT;
+	const int xw = blockIdx.x * Ring::COLUMNS, yw = (blockIdx.y * warps + warp) * Ring::OUT_ROWS; // the warp's first
+	const int x = xw + Ring::column(), y0 = yw + Ring::row();
 	const int z0 = blockIdx.z * a.zc, z1 = min(a.in.nz, z0 + a.zc);
 
 	// taps centred and zero-padded to 2 R + 1; an axis beyond the rank is the single tap 1
@@ -89,9 +88,9 @@ __global__ void __launch_bounds__(32 * WARPS, R >= 3 ? 2 : R == 2 ? 3 : 4)
 		taps[tid / K][tid % K] = make_float2(t, t);
 	}
 	__syncthreads();
-	if (y0 >= ny) return;
+	if (yw >= ny) return;
 	Ring ring;
-	ring.begin(smem, WARPS, warp, &source, a.in, xw, y0, z0 - R, z1 + R);
+	ring.begin(smem, warps, warp, &source, a.in, xw, yw, z0 - R, z1 + R);
 	const bool whole = x + OUT <= nx;
 	char* const column = a.dst + x * a.d_stride[0] + y0 * a.d_stride[1];
 
@@ -163,32 +162,43 @@ __global__ void __launch_bounds__(32 * WARPS, R >= 3 ? 2 : R == 2 ? 3 : 4)
 	}
 }
 
-template<int R, class Ring>
+template<int R, int LANES, class Ring>
 int launch_ring(const DevView& s, MarchArgs a, cudaStream_t st)
 {
-	constexpr size_t smem = Ring::bytes(WARPS);
+	const int warps = ring_warps<Ring>(a.in, WARPS);
+	const size_t smem = Ring::bytes(warps);
 	auto kernel = separable_march_kernel<R, Ring>;
 	IANE_GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
 		"separable: set shared memory size");
 	typename Ring::Source source{};
-	if constexpr (std::is_same_v<Ring, WarpRing<R>>) {
-		const int status = ring_map<R>(&source, s);
+	if constexpr (std::is_same_v<Ring, WarpRing<R, LANES>>) {
+		const int status = ring_map<R, LANES>(&source, s);
 		if (status) return status;
 	} else {
 		source = CopySource{s.ptr, s.stride[1], s.stride[2]};
 	}
-	const dim3 tiles((a.in.nx + kRingColumns - 1) / kRingColumns, (a.in.ny + OUT * WARPS - 1) / (OUT * WARPS));
+	const dim3 tiles = ring_tiles<Ring>(a.in, warps);
 	a.zc = ring_chunk(static_cast<long long>(tiles.x) * tiles.y, a.in.nz, R,
-		static_cast<long long>(R >= 3 ? 2 : R == 2 ? 3 : 4) * device_sm_count());
-	kernel<<<dim3(tiles.x, tiles.y, (a.in.nz + a.zc - 1) / a.zc), dim3(32, WARPS), smem, st>>>(source, a);
+		static_cast<long long>((R >= 3 ? 2 : R == 2 ? 3 : 4) * WARPS / warps) * device_sm_count());
+	kernel<<<dim3(tiles.x, tiles.y, (a.in.nz + a.zc - 1) / a.zc), dim3(32, warps), smem, st>>>(source, a);
 	IANE_GB_CUDA(cudaGetLastError(), "separable: launch");
 	return IANE_GB_OK;
+}
+
+template<int R, int LANES>
+int launch_lanes(const DevView& s, const MarchArgs& a, cudaStream_t st)
+{
+	return ring_supported(s) ? launch_ring<R, LANES, WarpRing<R, LANES>>(s, a, st)
+		: launch_ring<R, LANES, CopyRing<R, LANES>>(s, a, st);
 }
 
 template<int R>
 int launch(const DevView& s, const MarchArgs& a, cudaStream_t st)
 {
-	return ring_supported(s) ? launch_ring<R, WarpRing<R>>(s, a, st) : launch_ring<R, CopyRing<R>>(s, a, st);
+	// three taps are bound by memory, which idle lanes do not use (256 x 512 rows of 300: 57 us with 32 lanes side
+	// by side, 60 with 16), and nine taps' ring of 16 rows costs 4-byte copies a tenth (rows of 701: 485, 503)
+	const int most = R == 1 ? 3 : R == 4 && !ring_supported(s) ? 7 : 1 << 30;
+	return ring_narrow(a.in.nx, most) ? launch_lanes<R, 16>(s, a, st) : launch_lanes<R, 32>(s, a, st);
 }
 
 }  // namespace

@@ -1,6 +1,7 @@
 // A warp's own ring of input planes, for kernels whose warps march down z on their own (no block
-// barrier): 4 + 2 R rows of 128 columns with four more on either side, one TMA per plane, two planes
-// ahead of the one in use. Outside the image the TMA's zeros are the zero border. For clamp and
+// barrier). A lane has 4 columns and 4 rows; 32 lanes side by side make a warp's 128 x 4, or 16, two
+// such rows of them one above the other, its 64 x 8. A plane is the warp's rows and R more on either side, its
+// columns and four more on either side: one TMA per plane, two planes ahead of the one in use. Outside the image the TMA's zeros are the zero border. For clamp and
 // mirror a warp at an edge reads other rows in the place of those outside, and a lane at a row's end
 // takes the columns beyond it from its own four: a few selects. (Rewriting those cells in shared
 // memory after every copy is a chain of latencies that the edge warps' few neighbours do not hide:
@@ -13,11 +14,24 @@
 
 namespace iane_gb {
 
-constexpr int kRingOut = 4;                 // columns of a lane, and rows of a warp
-constexpr int kRingColumns = 32 * kRingOut; // columns of a warp
+constexpr int kRingOut = 4;                 // columns, and rows, of a lane
 constexpr int kRingStages = 3;
-constexpr int kRingGroups = 34;             // 16-byte groups of a row: the lanes' and one on either side
-constexpr int kRingFixes = 64;              // cells beyond the rows' ends in a plane: at most R x (4 + 2 R), R <= 4
+constexpr int kRingFixes = 64;              // cells beyond the rows' ends in a plane: at most R x (8 + 2 R), R <= 4
+
+// What the LANES side by side make of a warp.
+template<int R, int SIDE>
+struct RingShape {
+	static_assert(SIDE == 32 || SIDE == 16, "");
+	static constexpr int LANES = SIDE;
+	static constexpr int COLUMNS = LANES * kRingOut;
+	static constexpr int OUT_ROWS = 32 / LANES * kRingOut; // output rows
+	static constexpr int ROWS = OUT_ROWS + 2 * R;          // of a plane
+	static constexpr int GROUPS = LANES + 2;               // 16-byte groups of a row
+	// of this thread's lane: its group and first row, and the group at which row 0 of its window begins
+	static __device__ __forceinline__ int column() { return kRingOut * (LANES == 32 ? threadIdx.x : threadIdx.x & (LANES - 1)); }
+	static __device__ __forceinline__ int row() { return LANES == 32 ? 0 : kRingOut * ((threadIdx.x & 31) / LANES); }
+	static __device__ __forceinline__ int own() { return row() * GROUPS + (threadIdx.x & (LANES - 1)) + 1; }
+};
 
 // What a launch's warps share.
 struct RingArgs {
@@ -55,11 +69,12 @@ template<int R> __device__ __forceinline__ void ring_row(const float4* at, float
 	}
 }
 
-template<int R>
-struct WarpRing {
+template<int R, int LANES>
+struct WarpRing : RingShape<R, LANES> {
 	using Source = CUtensorMap;
-	static constexpr int ROWS = kRingOut + 2 * R;
-	static constexpr int PLANE = (ROWS * kRingGroups * 16 + 127) & ~127; // bytes; TMA writes to multiples of 128
+	using S = RingShape<R, LANES>;
+	static constexpr int WINDOW = kRingOut + 2 * R; // rows that a lane reads
+	static constexpr int PLANE = (S::ROWS * S::GROUPS * 16 + 127) & ~127; // bytes; TMA writes to multiples of 128
 	static constexpr int RING = kRingStages * PLANE;
 	// shared memory of a block of `warps` warps
 	static constexpr size_t bytes(int warps)
@@ -70,7 +85,7 @@ struct WarpRing {
 	unsigned char* ring;
 	uint64_t* bars;
 	int* fixes;             // ragged rows: cell << 16 | source, or -1
-	unsigned long long from; // edge: four bits per row, the row to read in its place
+	unsigned long long from; // edge: four bits per row of the lane's window, the one to read in its place
 	int x0, y0, z1;
 	int slot;
 	uint32_t parity;
@@ -95,26 +110,26 @@ struct WarpRing {
 		parity = 0;
 		ok = true;
 		const bool mapped = a.border != IANE_GB_BORDER_ZERO;
-		const bool edge_x = mapped && (x0 == 0 || x0 + kRingColumns + R > a.nx);
-		const bool edge_y = mapped && (y0 < R || y0 + kRingOut + R > a.ny);
+		const bool edge_x = mapped && (x0 == 0 || x0 + S::COLUMNS + R > a.nx);
+		const bool edge_y = mapped && (y0 < R || y0 + S::OUT_ROWS + R > a.ny);
 		edge = edge_x || edge_y;
 		clamp = a.border == IANE_GB_BORDER_CLAMP;
-		ragged = edge_x && a.nx % kRingOut != 0 && x0 + kRingColumns + R > a.nx;
-		left = mapped && x0 == 0 && lane == 0;
-		right = mapped && !ragged && x0 + kRingOut * (lane + 1) == a.nx;
+		ragged = edge_x && a.nx % kRingOut != 0 && x0 + S::COLUMNS + R > a.nx;
+		left = mapped && x0 + S::column() == 0;
+		right = mapped && !ragged && x0 + S::column() + kRingOut == a.nx;
 		if (lane == 0) {
 			for (int k = 0; k < kRingStages; ++k) mbar_init(&bars[k], 1);
 			fence_barrier_init();
 		}
 		from = 0;
-		for (int r = 0; r < ROWS; ++r) {
-			int row = y0 - R + r, to = r;
+		for (int r = 0; r < WINDOW; ++r) {
+			int row = y0 + S::row() - R + r, to = r;
 			// rows that no stored output reads stay
 			if (mapped && (row < 0 || row >= a.ny) && row < a.ny + R) {
 				int yi = 0;
 				map_coord(row, a.ny, a.border, yi);
-				to = yi - (y0 - R); // among the warp's rows, as the image has 16 or more
-				to = to < 0 ? 0 : to >= ROWS ? ROWS - 1 : to;
+				to = yi - (y0 + S::row() - R); // within the window, as the image has 16 or more
+				to = to < 0 ? 0 : to >= WINDOW ? WINDOW - 1 : to;
 			}
 			from |= static_cast<unsigned long long>(to) << (4 * r);
 		}
@@ -124,8 +139,8 @@ struct WarpRing {
 				int xi = 0;
 				map_coord(c, a.nx, a.border, xi);
 				const int to_at = c - x0 + kRingOut, from_at = xi - x0 + kRingOut;
-				const bool here = r < ROWS && to_at < 4 * kRingGroups && from_at >= 0;
-				fixes[i] = here ? (r * 4 * kRingGroups + to_at) << 16 | (r * 4 * kRingGroups + from_at) : -1;
+				const bool here = r < S::ROWS && to_at < 4 * S::GROUPS && from_at >= 0;
+				fixes[i] = here ? (r * 4 * S::GROUPS + to_at) << 16 | (r * 4 * S::GROUPS + from_at) : -1;
 			}
 		}
 		__syncwarp();
@@ -142,12 +157,12 @@ struct WarpRing {
 		if (!map_coord(z, a.nz, a.border, zi)) zi = z; // the zero border's plane: zeros
 		// order the warp's reads and edge writes of the slot before the copy into it
 		asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-		mbar_arrive_expect_tx(&bars[to], ROWS * kRingGroups * 16);
+		mbar_arrive_expect_tx(&bars[to], S::ROWS * S::GROUPS * 16);
 		tma_load_3d(ring + to * PLANE, map, x0 - kRingOut, y0 - R, zi, &bars[to]);
 	}
 
-	// Plane z, prepared: lane l's columns are group l + 1 of each row. The warp is done with the plane
-	// before it, whose slot takes another copy. All lanes.
+	// Plane z, prepared, for row(). The warp is done with the plane before it, whose slot takes another
+	// copy. All lanes.
 	__device__ __forceinline__ const float4* plane(const CUtensorMap* map, const RingArgs& a, int z)
 	{
 		__syncwarp();
@@ -172,17 +187,17 @@ struct WarpRing {
 		if (ragged) {
 			float* cells = reinterpret_cast<float*>(ring + slot * PLANE);
 #pragma unroll
-			for (int i = 0; i < R * ROWS; i += 32) {
+			for (int i = 0; i < R * S::ROWS; i += 32) {
 				const int e = fixes[i + (threadIdx.x & 31)];
 				if (e >= 0) cells[e >> 16] = cells[e & 0xffff];
 			}
 		}
 	}
 
-	// Row r of this lane's columns with R on either side, from plane(). EDGE: for warps with `edge`.
-	template<bool EDGE> __device__ __forceinline__ void row(const float4* rows, int r, float (&w)[kRingOut + 2 * R]) const
+	// Row r of the lane's window: its columns with R on either side, from plane(). EDGE: for warps with `edge`.
+	template<bool EDGE> __device__ __forceinline__ void read(const float4* rows, int r, float (&w)[kRingOut + 2 * R]) const
 	{
-		const float4* at = rows + (EDGE ? static_cast<int>(from >> (4 * r) & 15u) : r) * kRingGroups + (threadIdx.x & 31) + 1;
+		const float4* at = rows + (EDGE ? static_cast<int>(from >> (4 * r) & 15u) : r) * S::GROUPS + S::own();
 		ring_row<R>(at, w);
 		if constexpr (EDGE) {
 			// columns -1 - j and nx + j are columns j and nx - 1 - j under mirror
@@ -196,7 +211,7 @@ struct WarpRing {
 	}
 };
 
-// The same for rows that TMA cannot address: 4-byte cp.async, five per lane and row, from the columns and
+// The same for rows that TMA cannot address: 4-byte cp.async, lane by lane along each row, from the columns and
 // rows that the border rule names, so that no edge is left to the reader. (253 x 181 x 60, 7 separable
 // taps, mirror: 23 us; the block-wide kernel, which maps every cell of a plane on its own, 63.)
 struct CopySource {
@@ -204,18 +219,20 @@ struct CopySource {
 	long long s_row, s_plane;
 };
 
-template<int R>
-struct CopyRing {
+template<int R, int LANES>
+struct CopyRing : RingShape<R, LANES> {
 	using Source = CopySource;
-	static constexpr int ROWS = kRingOut + 2 * R;
-	static constexpr int PLANE = ROWS * kRingGroups * 16;
-	static constexpr int COPIES = (4 * kRingGroups + 31) / 32; // of a lane per row
+	using S = RingShape<R, LANES>;
+	static constexpr int PLANE = S::ROWS * S::GROUPS * 16;
+	static constexpr int COPIES = (4 * S::GROUPS + 31) / 32; // of a lane per row
+	static constexpr bool SPARE = S::ROWS < 16; // 15 names no row and stands for one that is not there
 	static constexpr size_t bytes(int warps) { return static_cast<size_t>(warps) * (kRingStages * PLANE + 32 * COPIES * 4); }
 	static constexpr bool edge = false;
 
 	unsigned char* ring;
 	int* columns;            // the source column of each, or -1
 	unsigned long long from; // four bits per row, the row to read in its place
+	uint32_t rows_in;        // without SPARE: a bit per row that is there
 	int y0, z1;
 	int slot;
 
@@ -229,12 +246,16 @@ struct CopyRing {
 		z1 = z_end;
 		slot = 0;
 		from = 0;
-		for (int r = 0; r < ROWS; ++r) {
+		rows_in = 0;
+		for (int r = 0; r < S::ROWS; ++r) {
 			int yi = 0;
 			const int at = y0 - R + r;
-			// rows and columns that no stored output reads stay out
-			const int to = at < a.ny + R && map_coord(at, a.ny, a.border, yi) ? yi - (y0 - R) : 15; // among the warp's rows
-			from |= static_cast<unsigned long long>(to < 0 || to >= ROWS ? 15 : to) << (4 * r);
+			// rows and columns that no stored output reads stay out; the others are among the plane's rows
+			const bool there = at < a.ny + R && map_coord(at, a.ny, a.border, yi);
+			const int to = yi - (y0 - R);
+			const bool use = there && to >= 0 && to < S::ROWS;
+			from |= static_cast<unsigned long long>(use ? to : 15) << (4 * r);
+			if (use) rows_in |= 1u << r;
 		}
 		for (int k = lane; k < 32 * COPIES; k += 32) {
 			int xi = 0;
@@ -264,12 +285,13 @@ struct CopyRing {
 			}
 			float* cells = reinterpret_cast<float*>(ring + to * PLANE) + lane;
 #pragma unroll 2
-			for (int r = 0; r < ROWS; ++r, cells += 4 * kRingGroups) {
+			for (int r = 0; r < S::ROWS; ++r, cells += 4 * S::GROUPS) {
 				const int f = static_cast<int>(from >> (4 * r) & 15u);
-				const char* row = plane + (f < ROWS ? y0 - R + f : 0) * s->s_row;
+				const bool there = SPARE ? f < S::ROWS : rows_in >> r & 1u;
+				const char* row = plane + (there ? y0 - R + f : 0) * s->s_row;
 #pragma unroll
 				for (int k = 0; k < COPIES; ++k) {
-					if (32 * k + lane < 4 * kRingGroups) cp_async4(cells + 32 * k, row + at[k], f < ROWS ? bytes[k] : 0);
+					if (32 * k + lane < 4 * S::GROUPS) cp_async4(cells + 32 * k, row + at[k], there ? bytes[k] : 0);
 				}
 			}
 		}
@@ -288,9 +310,9 @@ struct CopyRing {
 	// plane() brings the warp together.
 	__device__ __forceinline__ void prepare(const RingArgs&) { cp_async_wait<kRingStages - 2>(); }
 
-	template<bool EDGE> __device__ __forceinline__ void row(const float4* rows, int r, float (&w)[kRingOut + 2 * R]) const
+	template<bool EDGE> __device__ __forceinline__ void read(const float4* rows, int r, float (&w)[kRingOut + 2 * R]) const
 	{
-		ring_row<R>(rows + r * kRingGroups + (threadIdx.x & 31) + 1, w);
+		ring_row<R>(rows + r * S::GROUPS + S::own(), w);
 	}
 };
 
@@ -307,10 +329,23 @@ inline bool ring_supported(const DevView& s)
 		(s.ext[2] <= 1 || s.stride[2] >= s.stride[1] * s.ext[1]);
 }
 
-template<int R> int ring_map(CUtensorMap* map, const DevView& s)
+template<int R, int LANES> int ring_map(CUtensorMap* map, const DevView& s)
 {
 	return encode_tensor_map_f32(map, s.ptr, s.ext[0], s.ext[1], s.ext[2], s.stride[1],
-		s.ext[2] > 1 ? s.stride[2] : s.stride[1] * s.ext[1], 4 * kRingGroups, WarpRing<R>::ROWS);
+		s.ext[2] > 1 ? s.stride[2] : s.stride[1] * s.ext[1], 4 * RingShape<R, LANES>::GROUPS, RingShape<R, LANES>::ROWS);
+}
+
+// Warps of a block, one above the other: `most`, or as many as the rows need. The kernels of 32 lanes side
+// by side are compiled for `most`.
+template<class Shape> int ring_warps(const RingArgs& a, int most)
+{
+	return Shape::LANES == 32 ? most : min(most, (a.ny + Shape::OUT_ROWS - 1) / Shape::OUT_ROWS);
+}
+
+// Blocks of `warps` warps that cover the rows and columns.
+template<class Shape> dim3 ring_tiles(const RingArgs& a, int warps)
+{
+	return dim3((a.nx + Shape::COLUMNS - 1) / Shape::COLUMNS, (a.ny + Shape::OUT_ROWS * warps - 1) / (Shape::OUT_ROWS * warps));
 }
 
 }  // namespace iane_gb

@@ -266,6 +266,29 @@ def test_separable_volumes(cuda, shape, taps):
             assert not to_host(aside)[..., 0].any() and not to_host(apart)[..., 1::2].any()
 
 
+@pytest.mark.parametrize("shape,taps", [
+    ((9, 33, 97), (5, 3, 5)), ((40, 20, 101), (3, 3, 3)),    # 32 lanes side by side, rows that end inside a lane's columns
+    ((17, 45, 250), (7, 7, 5)), ((6, 19, 253), (9, 9, 9)),
+    ((300, 17, 64), (3, 3, 3)), ((7, 21, 65), (9, 3, 9)),    # 16, whole rows; one column in the next warp
+    ((5, 40, 449), (9, 9, 9)), ((4, 40, 513), (9, 9, 9)),    # up to a rule's limit and beyond it
+])
+def test_separable_volumes_by_lanes(cuda, shape, taps):
+    # as test_separable_volumes: rows as they are, and at TMA's pitch
+    rng = np.random.default_rng(sum(shape) + sum(taps))
+    src = rng.random(shape, dtype=np.float32) + np.float32(0.01)
+    tap_list = [rng.random(n, dtype=np.float32) + np.float32(0.1) for n in taps]
+    tol = (sum(taps) + 6) * 2.0 ** -24
+    wide = np.full((*shape[:-1], shape[-1] + 8 + -shape[-1] % 4), 7, np.float32)
+    wide[..., 4:4 + shape[-1]] = src
+    for border in ("clamp", "zero", "mirror"):
+        ref = np.zeros_like(src)
+        oracle.convolve_separable(src, tap_list, ref, border)
+        for g in (to_gpu(src), to_gpu(wide)[..., 4:4 + shape[-1]]):
+            out = empty_like_np(shape, np.float32)
+            iane_gb300.convolve_separable(g, [to_gpu(t) for t in tap_list], out, border)
+            assert float(np.max(np.abs(to_host(out) - ref) / ref)) <= tol, border
+
+
 def test_separable_strided_views(cuda):
     t = torch()
     rng = np.random.default_rng(8)

@@ -261,3 +261,24 @@ def test_planes_of_narrow_images(cuda, dtype, shape, radius):
         ref = np.zeros_like(src)
         oracle.morphology(src, ref, radius, op, border)
         assert run_gpu(src, radius, op, border).tobytes() == ref.tobytes(), (op, border)
+
+
+@pytest.mark.parametrize("shape,radius", [
+    ((9, 33, 100), 2), ((12, 20, 97), 1), ((8, 41, 250), 3),   # 32 lanes side by side
+    ((40, 17, 64), 1), ((7, 21, 65), 2), ((33, 64, 184), 3),   # 16
+])
+def test_volumes_by_lanes(cuda, shape, radius):
+    # rows that end inside a lane's columns and at them, at TMA's pitch
+    rng = np.random.default_rng(sum(shape) + radius)
+    wide = rng.standard_normal((*shape[:-1], shape[-1] + 8 + -shape[-1] % 4)).astype(np.float32)
+    for value in (np.nan, np.inf, 0.0):
+        wide[rng.random(wide.shape) < 0.03] = value
+    wide[: shape[0] // 2][rng.random((shape[0] // 2, *wide.shape[1:])) < 0.03] = -0.0
+    src = np.ascontiguousarray(wide[..., 4:4 + shape[-1]])
+    for op in ("erode", "dilate"):
+        for border in ("clamp", "zero", "mirror"):
+            ref = np.zeros_like(src)
+            oracle.morphology(src, ref, (radius,) * 3, op, border)
+            out = empty_like_np(shape, np.float32)
+            iane_gb300.morphology(to_gpu(wide)[..., 4:4 + shape[-1]], out, (radius,) * 3, op, border)
+            assert to_host(out).tobytes() == ref.tobytes(), (op, border)

@@ -15,6 +15,7 @@ extern "C" int chunk(long long columns, int nz, int r, long long slots, int* loo
 {
 	return iane_gb::ring_chunk(columns, nz, r, slots, looked);
 }
+extern "C" int narrow(int nx, int most) { return iane_gb::ring_narrow(nx, most); }
 """
 
 
@@ -46,3 +47,11 @@ def test_the_best_length_of_all(chunk, columns, nz, r, slots):
             break
     assert got == want
     assert looked.value <= 2 * math.sqrt(nz) + 2
+
+
+def test_no_half_of_a_warp_without_columns(tmp_path_factory):
+    narrow = compile_host(tmp_path_factory.mktemp("narrow"), SOURCE).narrow
+    for nx in range(16, 1200):
+        columns = 64 if narrow(nx, 1 << 30) else 128
+        assert -(-nx // columns) * columns - nx < 64, nx
+        assert narrow(nx, 3) == (narrow(nx, 1 << 30) and nx <= 192)
