@@ -345,7 +345,9 @@ __device__ __forceinline__ void plane_sums(float (&sum)[RY][RX], const float* ti
 // It pays for single planes (2560 x 1920 u8 9 x 9 clamp 36.9 -> 30.5 us, with the edge fix-up by rows);
 // where several planes follow it does not (64 x 256 x 256 under 15 x 15 x 7: 220.3 -> 222).
 // taps_resident: a single-plane caller's previous call left this kernel's taps in shared memory.
-template<int KX, int WX, int WY, int STAGE, bool SINGLE = false, int RX = kRX, int RY = kRY, bool FRESH = false>
+// EDGES: clamp and mirror borders too (without, TMA's zeros only).
+template<int KX, int WX, int WY, int STAGE, bool SINGLE = false, int RX = kRX, int RY = kRY, bool FRESH = false,
+	bool EDGES = true>
 __device__ __forceinline__ void conv_tile_sums(const CUtensorMap* tmap_ptr, const TileArgs& a, int x0, int y0, int z,
 	uint32_t& phases, uint64_t* bars, float (&acc)[RY][RX], bool taps_resident = false)
 {
@@ -456,7 +458,7 @@ __device__ __forceinline__ void conv_tile_sums(const CUtensorMap* tmap_ptr, cons
 	// out-of-image cells within (rx, ry) of the image -- the only ones stored outputs read --
 	// from the in-image cells the rule maps them to. Those lie inside the tile whenever
 	// nx > rx and ny > ry (the launcher's condition); any other cell keeps the TMA's zeros.
-	const bool fix_tile = STAGE != kTileCopy && a.border != IANE_GB_BORDER_ZERO &&
+	const bool fix_tile = EDGES && STAGE != kTileCopy && a.border != IANE_GB_BORDER_ZERO &&
 		!(x0 - G::RXA >= 0 && x0 - G::RXA + W <= a.nx && y0 - ry >= 0 && y0 + TY + ry <= a.ny);
 	for (int p = 0; p < nplanes; ++p) {
 		if constexpr (STAGE != kTileCopy) {
@@ -556,7 +558,7 @@ __device__ __forceinline__ uint64_t* tile_barriers(int ky, int kz)
 		tile_buffers(kz) * (plane_floats + psf_floats));
 }
 
-template<int KX, int WX, int WY, int STAGE, class Epi, bool SINGLE, int RX, int RY>
+template<int KX, int WX, int WY, int STAGE, class Epi, bool SINGLE, int RX, int RY, bool EDGES>
 __device__ __forceinline__ void conv_tile_block(const CUtensorMap& tmap, const TileArgs& a, const Epi& epi_in)
 {
 	if constexpr (STAGE != kTileCopy) {
@@ -575,7 +577,7 @@ __device__ __forceinline__ void conv_tile_block(const CUtensorMap& tmap, const T
 	const unsigned row = !ROTATE ? blockIdx.y : blockIdx.y == 0 ? gridDim.y - 1 : blockIdx.y - 1;
 	const int x0 = blockIdx.x * 32 * WX, y0 = row * 32 * WY;
 	float acc[RY][RX];
-	conv_tile_sums<KX, WX, WY, STAGE, SINGLE, RX, RY, SINGLE>(&tmap, a, x0, y0, blockIdx.z, phases,
+	conv_tile_sums<KX, WX, WY, STAGE, SINGLE, RX, RY, SINGLE, EDGES>(&tmap, a, x0, y0, blockIdx.z, phases,
 		tile_barriers<KX, WX, WY>(a.ky, a.kz), acc);
 	// the epilogue's state (pointers, Kahan sums) comes to life only after the sums
 	Epi epi = epi_in;
@@ -588,11 +590,11 @@ __device__ __forceinline__ void conv_tile_block(const CUtensorMap& tmap, const T
 	epi.finish();
 }
 
-template<int KX, int WX, int WY, int STAGE, class Epi, bool SINGLE, int RX, int RY>
+template<int KX, int WX, int WY, int STAGE, class Epi, bool SINGLE, int RX, int RY, bool EDGES>
 __global__ void __launch_bounds__(32 * WX * WY)
 	conv_tile_kernel(const __grid_constant__ CUtensorMap tmap, const TileArgs a, const __grid_constant__ Epi epi)
 {
-	conv_tile_block<KX, WX, WY, STAGE, Epi, SINGLE, RX, RY>(tmap, a, epi);
+	conv_tile_block<KX, WX, WY, STAGE, Epi, SINGLE, RX, RY, EDGES>(tmap, a, epi);
 }
 
 // The same held to the registers of BLOCKS blocks per SM.
@@ -600,16 +602,17 @@ template<int KX, int WX, int WY, int STAGE, class Epi, bool SINGLE, int RX, int 
 __global__ void __launch_bounds__(32 * WX * WY, BLOCKS)
 	conv_tile_kernel_held(const __grid_constant__ CUtensorMap tmap, const TileArgs a, const __grid_constant__ Epi epi)
 {
-	conv_tile_block<KX, WX, WY, STAGE, Epi, SINGLE, RX, RY>(tmap, a, epi);
+	conv_tile_block<KX, WX, WY, STAGE, Epi, SINGLE, RX, RY, true>(tmap, a, epi);
 }
 
 // Launch helper: grid = tiles over (x, y) and one block per output plane; RX x RY outputs per lane.
-template<int KX, int WX, int WY, int STAGE, bool SINGLE = false, int RX = kRX, int RY = kRY, int BLOCKS = 0, class Epi>
+template<int KX, int WX, int WY, int STAGE, bool SINGLE = false, int RX = kRX, int RY = kRY, int BLOCKS = 0, bool EDGES = true,
+	class Epi>
 int launch_tile(const CUtensorMap& map, const TileArgs& a, const Epi& epi, cudaStream_t stream)
 {
 	auto kernel = [] {
 		if constexpr (BLOCKS > 0) return conv_tile_kernel_held<KX, WX, WY, STAGE, Epi, SINGLE, RX, RY, BLOCKS>;
-		else return conv_tile_kernel<KX, WX, WY, STAGE, Epi, SINGLE, RX, RY>;
+		else return conv_tile_kernel<KX, WX, WY, STAGE, Epi, SINGLE, RX, RY, EDGES>;
 	}();
 	const int esize = (a.src_dtype == IANE_GB_U8 || a.src_dtype == IANE_GB_I8) ? 1 : 2;
 	const size_t smem = tile_smem_bytes<KX, WX, WY>(a.ky, a.kz, STAGE, esize);

@@ -205,6 +205,20 @@ def test_tile_staging(cuda, shape, kernel, dtype):
         assert float(np.max(np.abs(run_gpu(src, taps, np.float32, border) - ref) / ref)) <= tol, border
 
 
+@pytest.mark.parametrize("kernel", [(3, 9, 9), (3, 5, 17), (5, 21, 21), (1, 25, 25), (3, 3, 31)])
+@pytest.mark.parametrize("shape", [(7, 33, 40), (5, 70, 96), (1, 600, 612)])
+def test_small_volumes_with_a_zero_border(cuda, shape, kernel):
+    # TMA rows, tiles of 32 x 32: without the edge fix-up where the border is zero, with it elsewhere; n
+    # taps on positive data in FP32, one sum per kernel plane and those added up
+    rng = np.random.default_rng(sum(shape) + sum(kernel))
+    src = rng.random(shape, dtype=np.float32) + np.float32(0.01)
+    taps = rng.random(kernel, dtype=np.float32) + np.float32(0.1)
+    tol = (taps.size + 3) * 2.0 ** -24
+    for border in ("zero", "clamp"):
+        ref = run_oracle(src, taps, np.float32, border)
+        assert float(np.max(np.abs(run_gpu(src, taps, np.float32, border) - ref) / ref)) <= tol, border
+
+
 @pytest.mark.parametrize("border", ["clamp", "zero", "mirror"])
 @pytest.mark.parametrize("shape,taps", [((40,), (7,)), ((33, 70), (7, 7)), ((512, 512), (7, 7)), ((9, 30, 75), (5, 3, 7)),
                                        ((20, 20, 20), (9, 9, 9)), ((3, 5, 4), (7, 9, 11)), ((70, 90), (21, 3)),
