@@ -1,6 +1,7 @@
 // Batched Richardson-Lucy: plans, the work queue, the autotuned launch configuration, the
 // CUDA graph of a run and the C-ABI entry points iane_gb_rl_batch_*. See rl_batch.cuh for the
 // execution design.
+#include "batch_plan.h"
 #include "kernels.h"
 #include "rl_batch.cuh"
 
@@ -265,29 +266,6 @@ std::string cache_path()
 	return "iane_gb300_tune.txt";
 }
 
-// The batch signature: image count, a 64-bit FNV-1a hash of every (nx, ny, kx, ky), dtype, SMs.
-std::string tune_key(const std::vector<int>& nx, const std::vector<int>& ny, const std::vector<int>& kx,
-	const std::vector<int>& ky)
-{
-	uint64_t h = 1469598103934665603ull;
-	auto mix = [&](int v) {
-		for (int b = 0; b < 4; ++b) {
-			h ^= static_cast<uint64_t>((static_cast<uint32_t>(v) >> (8 * b)) & 0xffu);
-			h *= 1099511628211ull;
-		}
-	};
-	for (size_t i = 0; i < nx.size(); ++i) {
-		mix(nx[i]);
-		mix(ny[i]);
-		mix(kx[i]);
-		mix(ky[i]);
-	}
-	std::ostringstream k;
-	k << "rl2d-batch f32 images " << nx.size() << " shapes " << std::hex << h << std::dec << " sms "
-	  << device_sm_count();
-	return k.str();
-}
-
 void load_cache(TuneCache& c)
 {
 	if (c.loaded) return;
@@ -464,7 +442,7 @@ int autotune(iane_gb_rl_batch* b, cudaStream_t stream)
 	TuneCache& cache = tune_cache();
 	std::lock_guard<std::mutex> guard(cache.lock);
 	load_cache(cache);
-	const std::string key = tune_key(b->nx, b->ny, b->kx, b->ky);
+	const std::string key = tune_key(b->nx, b->ny, b->kx, b->ky, device_sm_count());
 	const auto hit = cache.choice.find(key);
 	const int max_bps = batch_blocks_per_sm(b->smem);
 	if (hit != cache.choice.end()) {

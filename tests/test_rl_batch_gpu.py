@@ -147,6 +147,28 @@ def test_autotune_cache_persists(cuda, tmp_path):
     assert len(cache.read_text().strip().splitlines()) == 1  # read from the cache, nothing re-measured
 
 
+def test_choices_of_another_version_are_not_taken(cuda, tmp_path):
+    # a line of the form written before the key had a version, whose order 0 and one CTA per SM were
+    # measured with another kernel: the batch is measured anew
+    cache = tmp_path / "tune.txt"
+    h = 1469598103934665603
+    for (ny, nx), k in zip([(40, 300), (200, 210), (64, 64)], (5, 15, 31)):
+        for v in (nx, ny, k, k):
+            for byte in v.to_bytes(4, "little"):
+                h = (h ^ byte) * 1099511628211 % 2 ** 64
+    sms = torch().cuda.get_device_properties(0).multi_processor_count
+    old = f"rl2d-batch f32 images 3 shapes {h:x} sms {sms} | 1.0 | 1 0 3"
+    cache.write_text(old + "\n")
+    env = dict(os.environ, IANE_GB_TUNE_CACHE=str(cache))
+    root = str(Path(__file__).resolve().parent.parent)
+    out = subprocess.run([sys.executable, "-c", AUTOTUNE_SCRIPT.format(root=root)], env=env, capture_output=True, text=True,
+                         timeout=600)
+    assert out.returncode == 0, out.stderr
+    lines = cache.read_text().strip().splitlines()
+    assert len(lines) == 2 and lines[0] == old
+    assert f"shapes {h:x} sms {sms} | " in lines[1]  # the same batch
+
+
 @pytest.mark.parametrize("grouping", [0, 1, 2, 3])
 def test_every_item_shape_matches_the_single_image_path(cuda, grouping):
     # the autotuner's item shapes (1, 2 or 4 tiles per item by PSF width) pinned one by one,
