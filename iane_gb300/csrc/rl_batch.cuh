@@ -22,14 +22,10 @@
 // captured on the first run and replayed while the views, scratch and parameters are unchanged.
 #pragma once
 
+#include "batch_plan.h"
 #include "rl.cuh"
 
-#include <vector>
-
 namespace iane_gb {
-
-// Tile edge of every work item (64 x 64 outputs; the body is 2 x 2 warps of 32 x 32).
-constexpr int kBatchTile = 64;
 
 // Device-side description of one image of the batch (128-byte aligned for the maps).
 struct alignas(128) BatchImage {
@@ -41,37 +37,6 @@ struct alignas(128) BatchImage {
 	int write_out_final;
 };
 static_assert(sizeof(BatchImage) % 16 == 0, "copied into shared memory in bulk");
-
-// `count` consecutive 64x64 tiles of one tile row of an image: the
-// item's shape is (64 count) x 64 (count is 1, 2 or 4, chosen per PSF size by the autotuner).
-struct alignas(16) BatchItem {
-	int image;
-	int x0, y0; // origin of the first tile
-	int count;
-	int image_tiles; // the image's 64x64 tiles (its completions per phase)
-	int kx, ky;
-	int reserved;
-};
-
-// Queues of one launch: at most one per PSF width (odd, 1 .. 31).
-constexpr int kBatchClasses = 16;
-constexpr int kBatchSmTable = 512;
-
-// One queue: items first .. first + count - 1 of a phase, taken phases times over, and what one
-// of them costs on average (any unit).
-struct BatchClass {
-	int first;
-	int count;
-	float cost;
-};
-
-// The queues of a launch and which of them the CTAs of each SM start on.
-struct BatchQueues {
-	int classes;
-	int sms;
-	BatchClass of[kBatchClasses];
-	unsigned char start[kBatchSmTable]; // by SM id, modulo sms
-};
 
 // Device words of a run, cleared before the launch: one counter per queue, the abort flag and
 // one completion counter per image.
