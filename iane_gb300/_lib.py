@@ -97,6 +97,7 @@ def lib() -> ctypes.CDLL:
     l.iane_gb_rl_batch_destroy.restype = ctypes.c_int
     sz, ll, f, i = ctypes.c_size_t, ctypes.c_longlong, ctypes.c_float, ctypes.c_int
     l.iane_gb_cnn_conv3.argtypes = [vp, i, vp, i, i, i, i, vp, vp, i, vp, vp, vp, i, vp, vp]
+    l.iane_gb_cnn_conv3_simt.argtypes = l.iane_gb_cnn_conv3.argtypes
     l.iane_gb_cnn_wgrad_scratch_bytes.argtypes = [i, i, i, i, i, i]
     l.iane_gb_cnn_wgrad_scratch_bytes.restype = sz
     l.iane_gb_cnn_conv3_wgrad.argtypes = [vp, i, vp, i, i, i, i, vp, i, vp, vp, vp, sz, vp]
@@ -111,7 +112,7 @@ def lib() -> ctypes.CDLL:
     l.iane_gb_cnn_tc_packed_bytes.restype = sz
     l.iane_gb_cnn_tc_pack.argtypes = [vp, i, i, i, vp, vp]
     l.iane_gb_cnn_conv3_tc.argtypes = [vp, i, vp, i, i, i, i, vp, vp, i, vp, vp, vp, i, vp]
-    for name in ("conv3", "conv3_wgrad", "flip", "pool2", "pool2_grad", "up2", "up2_grad", "mse", "adam", "tc_pack",
+    for name in ("conv3", "conv3_simt", "conv3_wgrad", "flip", "pool2", "pool2_grad", "up2", "up2_grad", "mse", "adam", "tc_pack",
                  "conv3_tc"):
         getattr(l, "iane_gb_cnn_" + name).restype = ctypes.c_int
     l.iane_gb_rl_destroy.argtypes = [vp]

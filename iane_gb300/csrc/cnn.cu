@@ -20,8 +20,8 @@
 //   pool2 / up2 and their gradients, mse (loss and gradient), adam (FP32 master weights)
 //
 // conv3 with BF16 output runs on the tensor cores (cnn_tc.cu) where the channels come in whole
-// octets. The rest -- FP32 outputs, whose sums keep plain FP32 arithmetic, odd channel counts
-// -- is a direct SIMT implementation: a CTA computes an 8x8x4 brick of output voxels for all
+// octets. The rest -- FP32 outputs, whose sums keep plain FP32 arithmetic, odd channel counts, and
+// whatever asks for it (conv3_simt) -- is a direct SIMT implementation: a CTA computes an 8x8x4 brick of output voxels for all
 // output channels, one voxel per thread with CO accumulators; input halo bricks and the
 // weights of four input channels are staged in shared memory per step, weights read as
 // warp-uniform 128-bit broadcasts.
@@ -449,6 +449,13 @@ int grid1(long long n)
 	return static_cast<int>(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
+bool conv3_arguments(const uint16_t* x0, int c0, const uint16_t* x1, int c1, int d, int h, int w, const uint16_t* weights,
+	int co, const uint16_t* y16, const float* y32, const float* residual)
+{
+	return x0 && c0 >= 1 && c1 >= 0 && (c1 == 0 || x1) && d >= 1 && h >= 1 && w >= 1 && weights && co >= 1 && co <= 64 &&
+		(y16 || y32) && !(residual && co != 1);
+}
+
 }  // namespace
 }  // namespace iane_gb
 
@@ -460,20 +467,28 @@ int iane_gb_cnn_conv3(const uint16_t* x0, int c0, const uint16_t* x1, int c1, in
 	const float* bias, int co, uint16_t* y16, float* y32, const float* residual, int act, const uint16_t* mask,
 	void* stream)
 {
-	if (!x0 || c0 < 1 || c1 < 0 || (c1 > 0 && !x1) || d < 1 || h < 1 || w < 1 || !weights || co < 1 || co > 64 ||
-	    (!y16 && !y32) || (residual && co != 1)) {
-		return fail(IANE_GB_INVALID_ARGUMENT, "cnn_conv3: bad arguments");
-	}
-	const cudaStream_t st = static_cast<cudaStream_t>(stream);
 	// Tensor cores: a BF16 result (the operands' products are exact and both paths sum in FP32, so
 	// the rounding to BF16 is what is left of the difference) of whole octets, whose unused slots
 	// would otherwise be read as data. 48 -> 16 channels on 64^3 voxels and the
 	// input gradient back to 48: 1068 us on the SIMT kernel, 115 us here.
-	if (y16 && !y32 && !residual && c0 % 8 == 0 && c1 % 8 == 0 && (c1 == 0 || c0 % 16 == 0) && co % 8 == 0 && aligned16(x0) &&
-	    aligned16(x1) && aligned16(y16) && aligned16(mask)) {
-		const int rc = launch_cnn_tc(x0, c0, x1, c1, d, h, w, weights, false, bias, co, y16, nullptr, nullptr, act, mask, st);
+	if (conv3_arguments(x0, c0, x1, c1, d, h, w, weights, co, y16, y32, residual) && y16 && !y32 && !residual &&
+	    c0 % 8 == 0 && c1 % 8 == 0 && (c1 == 0 || c0 % 16 == 0) && co % 8 == 0 && aligned16(x0) && aligned16(x1) &&
+	    aligned16(y16) && aligned16(mask)) {
+		const int rc = launch_cnn_tc(x0, c0, x1, c1, d, h, w, weights, false, bias, co, y16, nullptr, nullptr, act, mask,
+			static_cast<cudaStream_t>(stream));
 		if (rc != IANE_GB_UNSUPPORTED) return rc;
 	}
+	return iane_gb_cnn_conv3_simt(x0, c0, x1, c1, d, h, w, weights, bias, co, y16, y32, residual, act, mask, stream);
+}
+
+int iane_gb_cnn_conv3_simt(const uint16_t* x0, int c0, const uint16_t* x1, int c1, int d, int h, int w,
+	const uint16_t* weights, const float* bias, int co, uint16_t* y16, float* y32, const float* residual, int act,
+	const uint16_t* mask, void* stream)
+{
+	if (!conv3_arguments(x0, c0, x1, c1, d, h, w, weights, co, y16, y32, residual)) {
+		return fail(IANE_GB_INVALID_ARGUMENT, "cnn_conv3: bad arguments");
+	}
+	const cudaStream_t st = static_cast<cudaStream_t>(stream);
 	Conv3Args a{x0, x1, c0, c1, d, h, w, weights, bias, co, y16, y32, residual, act, mask, (w + BX - 1) / BX,
 		(h + BY - 1) / BY};
 	const dim3 grid(a.bricks_x * a.bricks_y, (d + BZ - 1) / BZ);

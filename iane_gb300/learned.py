@@ -140,10 +140,10 @@ class WarmStartNet:
 
     # -- operations ---------------------------------------------------------------------------
     def _conv(self, x0, c0, x1, c1, shape, weights, bias, co, y16=None, y32=None, residual=None, relu=True,
-              mask=None):
-        check(lib().iane_gb_cnn_conv3(_p(x0), c0, _p(x1), c1, shape[0], shape[1], shape[2], _p(weights), _p(bias),
-                                      co, _p(y16), _p(y32), _p(residual), 1 if relu else 0, _p(mask),
-                                      self._stream()))
+              mask=None, simt=False):
+        conv3 = lib().iane_gb_cnn_conv3_simt if simt else lib().iane_gb_cnn_conv3
+        check(conv3(_p(x0), c0, _p(x1), c1, shape[0], shape[1], shape[2], _p(weights), _p(bias), co, _p(y16), _p(y32),
+                    _p(residual), 1 if relu else 0, _p(mask), self._stream()))
 
     def _wgrad(self, b, x0, c0, x1, c1, shape, dy, co, name):
         scratch = b["wg"]
@@ -178,7 +178,12 @@ class WarmStartNet:
         """observed_norm: f32 tensor (D, H, W) = observed / mean(observed). Returns the
         (1, D, H, W) f32 output (normalised estimate); activations stay for backward().
         tensor_cores=True runs every convolution on the tcgen05 kernel (inference); the
-        default SIMT kernels are the ones the backward pass mirrors."""
+        default is the SIMT kernels, plain FP32 arithmetic throughout."""
+        return self._forward(observed_norm, sigma, "tensor" if tensor_cores else "simt")
+
+    def _forward(self, observed_norm, sigma: float, kernels: str):
+        """kernels: "tensor" (packed weights), "simt", or "train": as backward() computes its
+        convolutions, on the tensor cores where the output is BF16 and from plain weights."""
         shape = tuple(observed_norm.shape)
         b = self._buf(shape)
         s1 = shape
@@ -188,7 +193,7 @@ class WarmStartNet:
         b["res"][0].copy_(observed_norm)
         b["x16"][0, ..., 0].copy_(observed_norm)
         b["x16"][0, ..., 1].fill_(sigma / 3.0)
-        packs = self._packs() if tensor_cores else None
+        packs = self._packs() if kernels == "tensor" else None
 
         def c(name, x0, c0, x1, c1, s, co, y16=None, y32=None, residual=None, relu=True):
             if packs is not None:
@@ -197,7 +202,7 @@ class WarmStartNet:
                                                  1 if relu else 0, st))
             else:
                 self._conv(x0, c0, x1, c1, s, self.w16(name), self.bias(name), co, y16=y16, y32=y32,
-                           residual=residual, relu=relu)
+                           residual=residual, relu=relu, simt=kernels == "simt")
 
         c("e1a", b["x16"], 2, None, 0, s1, 16, y16=b["e1a"])
         c("e1b", b["e1a"], 16, None, 0, s1, 16, y16=b["e1b"])
@@ -393,7 +398,7 @@ def train(net: WarmStartNet, pairs, epochs=4, lr=2e-3, log=None, seed=0):
             observed, sigma, target, _ = pairs[i]
             mean = observed.double().mean().float().clamp_min(1e-6)
             net.zero_grad()
-            net.forward(observed / mean, sigma)
+            net._forward(observed / mean, sigma, "train")
             loss = net.loss_and_grad((target / mean).contiguous())
             net.backward(tuple(observed.shape))
             net.step(lr=lr * 0.25 ** (step / max(1, steps)))

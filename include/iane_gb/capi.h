@@ -356,6 +356,11 @@ int iane_gb_rl_batch_destroy(iane_gb_rl_batch* batch);
 int iane_gb_cnn_conv3(const uint16_t* x0, int c0, const uint16_t* x1, int c1, int d, int h, int w,
 	const uint16_t* weights, const float* bias, int co, uint16_t* y16, float* y32,
 	const float* residual, int act, const uint16_t* mask, void* stream);
+/* The same in plain FP32 arithmetic whatever the output (conv3 sums BF16 outputs of whole channel
+ * octets on the tensor cores, whose FP32 sums are cut off rather than rounded). */
+int iane_gb_cnn_conv3_simt(const uint16_t* x0, int c0, const uint16_t* x1, int c1, int d, int h, int w,
+	const uint16_t* weights, const float* bias, int co, uint16_t* y16, float* y32,
+	const float* residual, int act, const uint16_t* mask, void* stream);
 /* dw[co][ci][t] += sum_v dy[co](v) x[ci](v + t - 1); db[co] += sum_v dy[co](v) (FP32,
  * deterministic split-K through `scratch`). c0 a multiple of 8 when c1 > 0; x0, x1 16-byte
  * aligned. */

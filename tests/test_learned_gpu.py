@@ -515,3 +515,59 @@ def test_conv3_weight_gradient_on_tensor_cores(cuda, shape, c0, c1, co):
     for got, want, mag in zip((dw, db), *wants):
         err = (got.cpu().double() - want).abs()
         assert bool((err <= 1e-5 * mag + 2 ** -22 * want.abs() + 1e-30).all()), float((err - 1e-5 * mag).max())
+
+
+def _by_fp32(net):
+    """Replace the network's convolutions by ones that return FP32, which plain arithmetic sums,
+    rounded to BF16 here."""
+    import torch
+
+    def conv(x0, c0, x1, c1, shape, weights, bias, co, y16=None, y32=None, residual=None, relu=True, mask=None, **_):
+        out = y32 if y32 is not None else torch.empty((co, *shape), dtype=torch.float32, device=net.device)
+        _check(_lib().iane_gb_cnn_conv3(_p(x0), c0, _p(x1), c1, *shape, _p(weights), _p(bias), co, None, _p(out),
+                                        _p(residual), 1 if relu else 0, _p(mask), net._stream()))
+        if y16 is not None:
+            y16.view(-1)[: to_c8(out).numel()] = to_c8(out.to(torch.bfloat16)).view(-1)
+
+    net._conv = conv
+
+
+def test_the_default_forward_is_plain_fp32(cuda):
+    # what tensor_cores=True is compared with: bit for bit the sums that FP32 outputs have
+    import torch
+
+    from iane_gb300.learned import WarmStartNet
+
+    outs = []
+    for by_fp32 in (False, True):
+        net = WarmStartNet(cuda, seed=6)
+        gen = torch.Generator().manual_seed(4)
+        w0, b0 = net.offsets["head"]
+        net.master[w0:b0] = (torch.randn(b0 - w0, generator=gen) * 0.3).to(cuda)
+        net.p16.copy_(net.master.to(torch.bfloat16))
+        obs = (torch.rand((16, 36, 44), generator=gen, dtype=torch.float32) * 2.0).to(cuda)
+        if by_fp32:
+            _by_fp32(net)
+        outs.append(net.forward(obs, 1.5).cpu().clone())
+    assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("shape,c0,c1,co", [((3, 9, 10), 8, 0, 24), ((4, 6, 17), 24, 16, 32), ((2, 7, 8), 16, 0, 40),
+                                             ((3, 8, 9), 64, 0, 64)])
+def test_conv3_simt_sums_bf16_results_as_fp32_ones(cuda, shape, c0, c1, co):
+    # the SIMT kernels of up to 32 and up to 64 channels: BF16 results are FP32 ones rounded, under ReLU and a mask
+    import torch
+
+    gen = torch.Generator().manual_seed(c0 + co)
+    _, x0 = _act(gen, (c0,) + shape)
+    _, x1 = _act(gen, (max(c1, 8),) + shape)
+    mr, m = _act(gen, (co,) + shape)
+    _, w = _bf16_tensor(gen, (co, c0 + c1, 27), 0.2)
+    b = (torch.randn(co, generator=gen, dtype=torch.float32) * 0.1).to(cuda)
+    y16 = to_c8(torch.full((co,) + shape, 7.0, dtype=torch.bfloat16, device=cuda))
+    y32 = torch.empty((co,) + shape, dtype=torch.float32, device=cuda)
+    for out16, out32 in ((_p(y16), None), (None, _p(y32))):
+        _check(_lib().iane_gb_cnn_conv3_simt(_p(x0), c0, _p(x1) if c1 else None, c1, *shape, _p(w), _p(b), co, out16,
+                                             out32, None, 1, _p(m), None))
+    torch.cuda.synchronize()
+    assert torch.equal(from_c8(y16.cpu(), co), y32.cpu().to(torch.bfloat16))
