@@ -467,10 +467,10 @@ int iane_gb_cnn_conv3(const uint16_t* x0, int c0, const uint16_t* x1, int c1, in
 	const float* bias, int co, uint16_t* y16, float* y32, const float* residual, int act, const uint16_t* mask,
 	void* stream)
 {
-	// Tensor cores: a BF16 result (the operands' products are exact and both paths sum in FP32, so
-	// the rounding to BF16 is what is left of the difference) of whole octets, whose unused slots
+	// Tensor cores: a BF16 result (the operands' products are exact, both paths sum in FP32 and come
+	// equally near to the 64-bit sum, see TURNS in cnn_tc.cu) of whole octets, whose unused slots
 	// would otherwise be read as data. 48 -> 16 channels on 64^3 voxels and the
-	// input gradient back to 48: 1068 us on the SIMT kernel, 115 us here.
+	// input gradient back to 48: 1068 us on the SIMT kernel, 119 us here.
 	if (conv3_arguments(x0, c0, x1, c1, d, h, w, weights, co, y16, y32, residual) && y16 && !y32 && !residual &&
 	    c0 % 8 == 0 && c1 % 8 == 0 && (c1 == 0 || c0 % 16 == 0) && co % 8 == 0 && aligned16(x0) && aligned16(x1) &&
 	    aligned16(y16) && aligned16(mask)) {

@@ -93,7 +93,13 @@ __host__ __device__ __forceinline__ int weight_at(int n_rows, int ty, int h, int
 // What a launch stores: BF16, BF16 under a mask, or anything (FP32, a residual).
 constexpr int kPlain = 0, kMasked = 1, kFloat = 2;
 
-template<int N, int KIND>
+// TURNS: an accumulator takes one K step's nine MMAs and the epilogue adds the steps up in FP32
+// registers. The tensor cores cut their FP32 sums off, so that the error grows with the MMAs that one
+// accumulator takes; training's, whose sums were plain FP32 ones, comes no further from 64 bits this way
+// (of 1.35 million BF16 results of 96 random channels, 357 are not the nearest with plain FP32 sums, 697
+// with 54 MMAs in one accumulator, 175 so; of 16 channels, with nine either way, 70 and 76 of 0.68 million).
+// Each set starts with one MMA more: a training layer of 48 -> 16 channels on 64^3 voxels 183.7 -> 187 us.
+template<int N, int KIND, bool TURNS>
 __global__ void __launch_bounds__(THREADS) cnn_tc_conv_kernel(const __grid_constant__ CUtensorMap map0,
 	const __grid_constant__ CUtensorMap map1, const TcConvArgs a)
 {
@@ -207,15 +213,15 @@ __global__ void __launch_bounds__(THREADS) cnn_tc_conv_kernel(const __grid_const
 			if (a.packed && a.resident) wait(weights_in, 0);
 			int stage = 0;
 			uint32_t round = 0;
-			uint32_t i = 0; // tiles of this CTA so far
-			for (int tile = first; tile < a.tiles; tile += stride, ++i) {
-				const uint32_t set = i & 1;
-				if (i >= 2) wait(&drained[set], (i / 2 - 1) & 1);
-				tc::fence_after_sync();
-				const uint32_t d0 = tmem + set * SET, d1 = d0 + 3 * N;
+			uint32_t i = 0; // sets of accumulators of this CTA so far: a tile's, or with TURNS a step's
+			for (int tile = first; tile < a.tiles; tile += stride) {
 				for (int s = 0; s < a.steps; ++s) {
+					const bool opens = TURNS || s == 0;
+					const uint32_t set = i & 1;
+					if (opens && i >= 2) wait(&drained[set], (i / 2 - 1) & 1);
 					wait(&full[stage], round & 1);
 					tc::fence_after_sync();
+					const uint32_t d0 = tmem + set * SET, d1 = d0 + 3 * N;
 					const uint32_t a_base = smem_addr(smem + stage * stage_bytes);
 					const uint32_t b_base = a.resident ? smem_addr(resident + s * BB) : a_base + A_BYTES;
 					// input plane p reaches output plane 0 by tap tz = p and plane 1 by tz = p - 1; rows
@@ -228,12 +234,12 @@ __global__ void __launch_bounds__(THREADS) cnn_tc_conv_kernel(const __grid_const
 							const uint32_t row = b_base + static_cast<uint32_t>(ty) * 2 * HALF;
 							auto taps = [&](int tz) { return tc::smem_desc(row + static_cast<uint32_t>((2 - tz) * 3 * N * 16), HALF, 128); };
 							if (p == 0) {
-								tc::mma_bf16(d0, ad, taps(0), idesc3, s > 0 || ty > 0);
+								tc::mma_bf16(d0, ad, taps(0), idesc3, !opens || ty > 0);
 							} else if (p == 3) {
 								tc::mma_bf16(d1, ad, taps(2), idesc3, true);
 							} else if (p == 1 && ty == 0) {
-								// the first step starts plane 1's accumulators here
-								if (s > 0) {
+								// a set's first step starts plane 1's accumulators here
+								if (!opens) {
 									tc::mma_bf16(d0, ad, taps(1), idesc6, true);
 								} else {
 									tc::mma_bf16(d0, ad, taps(1), idesc3, true);
@@ -249,8 +255,11 @@ __global__ void __launch_bounds__(THREADS) cnn_tc_conv_kernel(const __grid_const
 						stage = 0;
 						++round;
 					}
+					if (TURNS || s + 1 == a.steps) {
+						tc::commit(&ready[set]);
+						++i;
+					}
 				}
-				tc::commit(&ready[set]);
 			}
 			// no MMA may be in flight when the CTA gives its memory back
 			if (i > 0) wait(&ready[(i - 1) & 1], ((i - 1) / 2) & 1);
@@ -263,35 +272,35 @@ __global__ void __launch_bounds__(THREADS) cnn_tc_conv_kernel(const __grid_const
 		const long long plane = static_cast<long long>(a.h) * a.w, vol = plane * a.d;
 		const uint32_t lane_base = static_cast<uint32_t>(32 * warp) << 16;
 		uint32_t i = 0;
-		for (int tile = first; tile < a.tiles; tile += stride, ++i) {
-			const uint32_t set = i & 1;
+		for (int tile = first; tile < a.tiles; tile += stride) {
 			int x0, y0, z0;
 			origin(tile, x0, y0, z0);
 			const int x = x0 - 1 + (r & 15), y = y0 + (r >> 4);
 			const bool valid = (r & 15) >= 1 && (r & 15) <= OUT_X && x < a.w && y < a.h;
 			const long long v0 = z0 * plane + static_cast<long long>(y) * a.w + x;
-			wait(&ready[set], (i / 2) & 1);
-#pragma unroll 1
-			for (int q = 0; q < BZ * (N / 16); ++q) {
-				__syncwarp(); // tcgen05.ld is warp-collective: lanes come from the wait or from `continue`
-				tc::fence_after_sync();
+			// group q of 16 channels of a plane: the sum over the x taps
+			auto group = [&](uint32_t set, int q, float (&o)[16]) {
 				const int zb = q / (N / 16), j = q % (N / 16);
-				const long long v = zb ? v0 + plane : v0;
+				__syncwarp(); // tcgen05.ld is warp-collective: lanes come from the wait or from store()
+				tc::fence_after_sync();
 				float d0[16], d1[16], d2[16];
 				const uint32_t col = tmem + lane_base + set * SET + static_cast<uint32_t>(zb * 3 * N + 16 * j);
 				tc::ld_32x32b_x16x3(col, col + N, col + 2 * N, d0, d1, d2);
 				if (q == BZ * (N / 16) - 1) {
-					// the set has been read: the next tile's MMAs may have it
+					// the set has been read: its next MMAs may have it
 					tc::fence_before_sync();
 					__syncwarp();
 					if (lane == 0) mbar_arrive(&drained[set]);
 				}
-				float o[16];
 #pragma unroll
 				for (int k = 0; k < 16; ++k) {
 					o[k] = __shfl_up_sync(0xffffffffu, d0[k], 1) + d1[k] + __shfl_down_sync(0xffffffffu, d2[k], 1);
 				}
-				if (!valid || z0 + zb >= a.d) continue;
+			};
+			auto store = [&](int q, float (&o)[16]) {
+				const int zb = q / (N / 16), j = q % (N / 16);
+				const long long v = zb ? v0 + plane : v0;
+				if (!valid || z0 + zb >= a.d) return;
 				const int c0 = co0 + 16 * j;
 #pragma unroll
 				for (int k = 0; k < 16; k += 4) {
@@ -341,6 +350,31 @@ __global__ void __launch_bounds__(THREADS) cnn_tc_conv_kernel(const __grid_const
 						*reinterpret_cast<uint4*>(a.y16 + at) = make_uint4(u[0], u[1], u[2], u[3]);
 					}
 				}
+			};
+			if constexpr (TURNS) {
+				float sum[BZ * (N / 16)][16];
+				for (int s = 0; s < a.steps; ++s, ++i) {
+					wait(&ready[i & 1], (i / 2) & 1);
+#pragma unroll
+					for (int q = 0; q < BZ * (N / 16); ++q) {
+						float o[16];
+						group(i & 1, q, o);
+#pragma unroll
+						for (int k = 0; k < 16; ++k) sum[q][k] = s > 0 ? sum[q][k] + o[k] : o[k];
+					}
+				}
+#pragma unroll
+				for (int q = 0; q < BZ * (N / 16); ++q) store(q, sum[q]);
+			} else {
+				const uint32_t set = i & 1;
+				wait(&ready[set], (i / 2) & 1);
+#pragma unroll 1
+				for (int q = 0; q < BZ * (N / 16); ++q) {
+					float o[16];
+					group(set, q, o);
+					store(q, o);
+				}
+				++i;
 			}
 		}
 	}
@@ -378,8 +412,9 @@ int n_tiles_of(int co) { return (co + n_of(co) - 1) / n_of(co); }
 template<int N>
 int launch(const CUtensorMap& m0, const CUtensorMap& m1, TcConvArgs a, cudaStream_t st)
 {
-	const auto kernel = a.y32 || a.residual ? cnn_tc_conv_kernel<N, kFloat>
-		: a.mask ? cnn_tc_conv_kernel<N, kMasked> : cnn_tc_conv_kernel<N, kPlain>;
+	// plain weights are training's, whose results are BF16; packed ones inference's, without a mask
+	const auto kernel = !a.packed ? a.mask ? cnn_tc_conv_kernel<N, kMasked, true> : cnn_tc_conv_kernel<N, kPlain, true>
+		: a.y32 || a.residual ? cnn_tc_conv_kernel<N, kFloat, false> : cnn_tc_conv_kernel<N, kPlain, false>;
 	// weights resident beside two or three input stages, or a stage of both at a time
 	const size_t weights = static_cast<size_t>(a.steps) * b_bytes(N);
 	// CTAs per SM are bounded by TMEM (512 columns per SM): ask for enough shared memory that

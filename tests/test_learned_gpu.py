@@ -571,3 +571,23 @@ def test_conv3_simt_sums_bf16_results_as_fp32_ones(cuda, shape, c0, c1, co):
                                              out32, None, 1, _p(m), None))
     torch.cuda.synchronize()
     assert torch.equal(from_c8(y16.cpu(), co), y32.cpu().to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("c0,c1,co", [(64, 32, 32), (64, 0, 64)])
+def test_conv3_on_tensor_cores_is_as_near_as_plain_fp32(cuda, c0, c1, co):
+    # of the BF16 results, no more miss the one nearest to the 64-bit sum than with plain FP32 arithmetic
+    import torch
+
+    shape = (16, 40, 44)
+    gen = torch.Generator().manual_seed(c0 + co)
+    x0r, x0 = _act(gen, (c0,) + shape)
+    x1r, x1 = _act(gen, (max(c1, 8),) + shape)
+    wr, w = _bf16_tensor(gen, (co, c0 + c1, 27), 0.1)
+    nearest = bf16_round(conv3(torch.cat([x0r, x1r[:c1]], 0) if c1 else x0r, wr))
+    missed = []
+    for f in (_lib().iane_gb_cnn_conv3_simt, _lib().iane_gb_cnn_conv3):
+        y = to_c8(torch.zeros((co,) + shape, dtype=torch.bfloat16, device=cuda))
+        _check(f(_p(x0), c0, _p(x1) if c1 else None, c1, *shape, _p(w), None, co, _p(y), None, None, 0, None, None))
+        torch.cuda.synchronize()
+        missed.append(int((from_c8(y.cpu(), co).double() != nearest).sum()))
+    assert missed[1] <= missed[0], missed

@@ -1,5 +1,5 @@
 """Tensor-memory loads (tcgen05.ld .sync.aligned) need their whole warp together. In the sources: a
-loop body that lanes can leave early (`continue`) brings the warp together again (__syncwarp) before
+loop body that lanes can leave early (`continue`, or `return` from a lambda in it) brings the warp together again (__syncwarp) before
 a load in it."""
 from __future__ import annotations
 
@@ -29,7 +29,7 @@ def offences(text):
     text = re.sub(r"//[^\n]*", lambda m: " " * len(m.group()), text)
     for call in CALL.finditer(text):
         for start, end in loops_around(text, call.start()):
-            if "continue;" in text[start:end] and "__syncwarp()" not in text[start:call.start()]:
+            if re.search(r"\b(continue|return);", text[start:end]) and "__syncwarp()" not in text[start:call.start()]:
                 yield text[:call.start()].count("\n") + 1
 
 
