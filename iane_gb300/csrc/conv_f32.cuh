@@ -73,11 +73,13 @@ int launch_f32_kx(const DevView& src, const DevView& kernel, const DevView& dst,
 	// schedules the sums of some widths worse (64 x 64 x 16: 9 x 9 x 5 24.9 -> 22.8 us, 17 x 17 x 3 33 -> 32, 25 x 25 x 3
 	// 20% less, 31 x 31 x 3 94 -> 82; 21 x 21 x 3 would go from 45.6 to 47.5, up to seven wide nothing changes).
 	constexpr bool EDGES = KX < 9 || KX == 21;
+	if constexpr (KX <= 9) {
+		if (five && stage == kTileCopy) return launch_tile<KX, 2, 2, kTileCopy, false, kRX, kRY, 5>(map, a, epi, stream);
+	}
 	if (stage == kTileCopy) {
 		// up to 15 wide held to seven blocks per SM, as TMA staging has them by itself (2047 x 2049 bf16
 		// 9 x 9 mirror: 41 -> 33 us)
 		return single ? launch_tile<KX, 2, 2, kTileCopy, true, kRX, kRY, KX <= 15 ? 7 : 0>(map, a, epi, stream)
-			: five ? launch_tile<KX, 2, 2, kTileCopy, false, kRX, kRY, KX <= 9 ? 5 : 0>(map, a, epi, stream)
 			: big ? launch_tile<KX, 2, 2, kTileCopy, false, RX, RY>(map, a, epi, stream)
 			: launch_tile<KX, 1, 1, kTileCopy>(map, a, epi, stream);
 	}
@@ -91,8 +93,10 @@ int launch_f32_kx(const DevView& src, const DevView& kernel, const DevView& dst,
 		const int status =
 			encode_tensor_map_f32(&map, src.ptr, src.ext[0], src.ext[1], src.ext[2], row, plane, box_w, box_h);
 		if (status) return status;
+		if constexpr (KX <= 9) {
+			if (five) return launch_tile<KX, 2, 2, kTileTma, false, kRX, kRY, 5>(map, a, epi, stream);
+		}
 		return single ? launch_tile<KX, 2, 2, kTileTma, true>(map, a, epi, stream)
-			: five ? launch_tile<KX, 2, 2, kTileTma, false, kRX, kRY, KX <= 9 ? 5 : 0>(map, a, epi, stream)
 			: big ? launch_tile<KX, 2, 2, kTileTma, false, RX, RY>(map, a, epi, stream)
 			: border == IANE_GB_BORDER_ZERO ? launch_tile<KX, 1, 1, kTileTma, false, kRX, kRY, 0, EDGES>(map, a, epi, stream)
 			: launch_tile<KX, 1, 1, kTileTma>(map, a, epi, stream);

@@ -344,17 +344,15 @@ __device__ __forceinline__ void plane_sums(float (&sum)[RY][RX], const float* ti
 // FRESH: no call before this one in the block (its buffers are free): the tile comes while the taps do.
 // It pays for single planes (2560 x 1920 u8 9 x 9 clamp 36.9 -> 30.5 us, with the edge fix-up by rows);
 // where several planes follow it does not (64 x 256 x 256 under 15 x 15 x 7: 220.3 -> 222).
-// taps_resident: a single-plane caller's previous call left this kernel's taps in shared memory.
 // EDGES: clamp and mirror borders too (without, TMA's zeros only).
 template<int KX, int WX, int WY, int STAGE, bool SINGLE = false, int RX = kRX, int RY = kRY, bool FRESH = false,
 	bool EDGES = true>
 __device__ __forceinline__ void conv_tile_sums(const CUtensorMap* tmap_ptr, const TileArgs& a, int x0, int y0, int z,
-	uint32_t& phases, uint64_t* bars, float (&acc)[RY][RX], bool taps_resident = false)
+	uint32_t& phases, uint64_t* bars, float (&acc)[RY][RX])
 {
 	static_assert(RX % 4 == 0 && RX * RY == kRX * kRY && 32 % RX == 0, "a lane owns 32 outputs of a 32 x 32 warp tile");
 	constexpr int LX = 32 / RX; // lanes along x in a warp
 	using G = TileGeom<KX>;
-	constexpr int TX = 32 * WX;
 	constexpr int TY = 32 * WY;
 	constexpr int P = TileWidth<KX, WX>::P;
 	constexpr int W = TileWidth<KX, WX>::W;
@@ -443,7 +441,7 @@ __device__ __forceinline__ void conv_tile_sums(const CUtensorMap* tmap_ptr, cons
 		if (nplanes > 1) issue(1);
 	};
 	if constexpr (FRESH) issue_first();
-	if (nplanes > 0 && !(SINGLE && taps_resident)) load_taps(0);
+	if (nplanes > 0) load_taps(0);
 	if (nplanes > 1) load_taps(1);
 	__syncthreads(); // taps visible; every lane is done with the previous tile's buffers
 	if constexpr (!FRESH) issue_first();
