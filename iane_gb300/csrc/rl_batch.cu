@@ -198,7 +198,7 @@ struct iane_gb_rl_batch {
 	int group = 0;                         // item shapes by PSF width (autotuned, tiles_per_item)
 	iane_gb::BatchImage* d_images = nullptr;
 	iane_gb::InitDesc* d_init = nullptr;
-	size_t parts_off = 0, sync_off = 0, scratch_bytes = 0;
+	size_t sync_off = 0, scratch_bytes = 0; // the images end at sync_off
 	cudaStream_t capture = nullptr;
 	cudaGraphExec_t exec = nullptr;
 	std::string key;
@@ -394,7 +394,7 @@ int autotune(iane_gb_rl_batch* b, cudaStream_t stream)
 	std::vector<InitDesc> idesc;
 	int st = fill_images(b, obs.data(), nullptr, 1e-6f, base, host, idesc);
 	if (st) return release(st);
-	IANE_GB_CUDA(cudaMemset(base, 0, b->parts_off), "autotune: clear images");
+	IANE_GB_CUDA(cudaMemset(base, 0, b->sync_off), "autotune: clear images");
 	if (cudaMemcpy(d_images, host.data(), n * sizeof(BatchImage), cudaMemcpyHostToDevice) != cudaSuccess) {
 		return release(cuda_fail(cudaGetLastError(), "autotune: upload"));
 	}
@@ -517,8 +517,6 @@ int iane_gb_rl_batch_prepare(const iane_gb_view* psfs, int count, const int32_t*
 		b->img_bytes.push_back(bytes);
 		off += 2 * bytes;
 	}
-	b->parts_off = off;
-	off += align_up(static_cast<size_t>(count) * sizeof(float));
 	b->sync_off = off;
 	off += align_up(sync_bytes(count));
 	b->scratch_bytes = off + kAlignB;

@@ -219,3 +219,23 @@ def test_queues_of_a_run_match_the_single_image_path(cuda, shapes, ks, mode):
         rl.close()
     iane_gb300.device_status()
     batch.close()
+
+
+@pytest.mark.parametrize("shapes", [[(5, 7)], [(64, 64)] * 3, [(10, 300)] * 70])
+def test_scratch_is_the_images_and_the_counters(cuda, shapes):
+    # two work images each, and words for the queues, the abort flag and every image's counter, in whole
+    # 256 bytes; a run takes exactly that and refuses a byte less
+    t = torch()
+    batch = iane_gb300.RichardsonLucyBatch([to_gpu(gaussian((3, 3), (0.8, 0.8)))] * len(shapes), shapes)
+    up = lambda n: -(-n // 256) * 256  # noqa: E731
+    images = sum(2 * up(-(-nx // 4) * 4 * ny * 4) for ny, nx in shapes)
+    assert batch.scratch_bytes == images + up(4 * (len(shapes) + 17)) + 256
+    obs = [t.full(s, 3.0, device="cuda") for s in shapes]
+    outs = [t.empty(s, device="cuda") for s in shapes]
+    scratch = t.empty(batch.scratch_bytes, dtype=t.uint8, device="cuda")
+    batch.run(obs, outs, 2, 1e-6, init=1, scratch=scratch)
+    assert all(bool(t.isfinite(o).all()) for o in outs)
+    with pytest.raises(iane_gb300.IaneError):
+        batch.run(obs, outs, 2, 1e-6, init=1, scratch=scratch[:-1])
+    iane_gb300.device_status()
+    batch.close()
