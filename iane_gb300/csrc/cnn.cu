@@ -449,6 +449,10 @@ int grid1(long long n)
 	return static_cast<int>(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
+// Bricks of a volume d deep; conv3 refuses those beyond a grid's limit, whichever kernel they would take.
+constexpr unsigned kMaxGridY = 65535;
+unsigned conv3_planes(int d) { return (static_cast<unsigned>(d) + BZ - 1) / BZ; }
+
 bool conv3_arguments(const uint16_t* x0, int c0, const uint16_t* x1, int c1, int d, int h, int w, const uint16_t* weights,
 	int co, const uint16_t* y16, const float* y32, const float* residual)
 {
@@ -471,8 +475,8 @@ int iane_gb_cnn_conv3(const uint16_t* x0, int c0, const uint16_t* x1, int c1, in
 	// equally near to the 64-bit sum, see TURNS in cnn_tc.cu) of whole octets, whose unused slots
 	// would otherwise be read as data. 48 -> 16 channels on 64^3 voxels and the
 	// input gradient back to 48: 1068 us on the SIMT kernel, 119 us here.
-	if (conv3_arguments(x0, c0, x1, c1, d, h, w, weights, co, y16, y32, residual) && y16 && !y32 && !residual &&
-	    c0 % 8 == 0 && c1 % 8 == 0 && (c1 == 0 || c0 % 16 == 0) && co % 8 == 0 && aligned16(x0) && aligned16(x1) &&
+	if (conv3_arguments(x0, c0, x1, c1, d, h, w, weights, co, y16, y32, residual) && conv3_planes(d) <= kMaxGridY &&
+	    y16 && !y32 && !residual && c0 % 8 == 0 && c1 % 8 == 0 && (c1 == 0 || c0 % 16 == 0) && co % 8 == 0 && aligned16(x0) && aligned16(x1) &&
 	    aligned16(y16) && aligned16(mask)) {
 		const int rc = launch_cnn_tc(x0, c0, x1, c1, d, h, w, weights, false, bias, co, y16, nullptr, nullptr, act, mask,
 			static_cast<cudaStream_t>(stream));
@@ -491,8 +495,8 @@ int iane_gb_cnn_conv3_simt(const uint16_t* x0, int c0, const uint16_t* x1, int c
 	const cudaStream_t st = static_cast<cudaStream_t>(stream);
 	Conv3Args a{x0, x1, c0, c1, d, h, w, weights, bias, co, y16, y32, residual, act, mask, (w + BX - 1) / BX,
 		(h + BY - 1) / BY};
-	const dim3 grid(a.bricks_x * a.bricks_y, (d + BZ - 1) / BZ);
-	if (grid.y > 65535) return fail(IANE_GB_UNSUPPORTED, "cnn_conv3: volume too deep");
+	const dim3 grid(a.bricks_x * a.bricks_y, conv3_planes(d));
+	if (grid.y > kMaxGridY) return fail(IANE_GB_UNSUPPORTED, "cnn_conv3: volume too deep");
 	if (co <= 4) {
 		conv3_kernel<4><<<grid, NT, 0, st>>>(a);
 	} else if (co <= 16) {

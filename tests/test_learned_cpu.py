@@ -37,3 +37,15 @@ def test_weights_file_round_trip(tmp_path):
     path.write_bytes(bytes(path.read_bytes()[:100]))
     with pytest.raises(ValueError):
         other.load(path)
+
+
+def test_conv3_refuses_too_deep_a_volume_for_every_kernel():
+    # 4 planes to a brick, 65535 bricks: refused before any CUDA call, for channels in whole octets (the
+    # tensor cores') as for others; the pointers are never read
+    from iane_gb300 import _lib
+
+    lib = _lib.lib()
+    for conv3 in (lib.iane_gb_cnn_conv3, lib.iane_gb_cnn_conv3_simt):
+        for c0, co in ((16, 16), (3, 5)):
+            status = conv3(16, c0, None, 0, 4 * 65535 + 1, 1, 1, 16, None, co, 16, None, None, 0, None, None)
+            assert status == -2 and "too deep" in _lib.last_error()
