@@ -591,3 +591,35 @@ def test_conv3_on_tensor_cores_is_as_near_as_plain_fp32(cuda, c0, c1, co):
         torch.cuda.synchronize()
         missed.append(int((from_c8(y.cpu(), co).double() != nearest).sum()))
     assert missed[1] <= missed[0], missed
+
+
+@pytest.mark.parametrize("shape,c0,c1,co", [((3, 5, 17), 40, 0, 17), ((4, 8, 16), 16, 8, 16)])
+def test_conv3_weight_gradient_of_unaligned_dy(cuda, shape, c0, c1, co):
+    # a dy that 16-byte copies cannot read takes the SIMT kernel: 1e-5 of the terms' magnitudes, and the
+    # rounding of the result, as test_conv3_weight_gradient
+    import torch
+
+    gen = torch.Generator().manual_seed(c0 + co)
+    x0r, x0 = _act(gen, (c0,) + shape)
+    x1r, x1 = _act(gen, (max(c1, 8),) + shape)
+    dyr, dy = _act(gen, (co,) + shape)
+    room = torch.zeros(dy.numel() + 8, dtype=torch.bfloat16, device=cuda)
+    apart = room[1:1 + dy.numel()]
+    apart.copy_(dy.view(-1))
+    assert apart.data_ptr() % 16 == 2
+    inp = torch.cat([x0r, x1r[:c1]], 0) if c1 else x0r
+    wants = []
+    for a, b in ((inp, dyr), (inp.abs(), dyr.abs())):
+        p = torch.nn.functional.pad(a, (1, 1, 1, 1, 1, 1))
+        d, h, w = shape
+        rows = [p[:, t // 9:t // 9 + d, t // 3 % 3:t // 3 % 3 + h, t % 3:t % 3 + w].reshape(c0 + c1, -1) for t in range(27)]
+        wants.append((torch.stack([b.reshape(co, -1) @ r.T for r in rows], 2), b.reshape(co, -1).sum(1)))
+    dw = torch.zeros((co, c0 + c1, 27), dtype=torch.float32, device=cuda)
+    db = torch.zeros(co, dtype=torch.float32, device=cuda)
+    scratch = torch.empty(int(_lib().iane_gb_cnn_wgrad_scratch_bytes(c0, c1, *shape, co)), dtype=torch.uint8, device=cuda)
+    _check(_lib().iane_gb_cnn_conv3_wgrad(_p(x0), c0, _p(x1) if c1 else None, c1, *shape, _p(apart), co, _p(dw), _p(db),
+                                          _p(scratch), scratch.numel(), None))
+    torch.cuda.synchronize()
+    for got, want, mag in zip((dw, db), *wants):
+        err = (got.cpu().double() - want).abs()
+        assert bool((err <= 1e-5 * mag + 2 ** -22 * want.abs() + 1e-30).all()), float((err - 1e-5 * mag).max())
