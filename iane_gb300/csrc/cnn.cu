@@ -553,7 +553,7 @@ int iane_gb_cnn_conv3_wgrad(const uint16_t* x0, int c0, const uint16_t* x1, int 
 	a.chunks = static_cast<int>(chunks);
 	const cudaStream_t st = static_cast<cudaStream_t>(stream);
 	// Tensor cores (cnn_wgrad.cu) wherever dy can be read by 16-byte copies. 48 -> 16 channels on 64^3
-	// voxels: 1340 us on the SIMT kernel, about 60 here, with the smaller error; 64 -> 64 channels on
+	// voxels: 1340 us on the SIMT kernel, about 70 here, with the smaller error; 64 -> 64 channels on
 	// 11 x 11 x 6 voxels (all three passes of the layer) 766 and 145 us.
 	if (aligned16(dy)) {
 		const int rc = launch_cnn_wgrad_tc(x0, c0, x1, c1, d, h, w, dy, co, dw, db, a.partial, a.chunks, st);

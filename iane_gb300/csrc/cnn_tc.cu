@@ -35,8 +35,8 @@
 // issues MMAs into one of two TMEM accumulator sets, four warps empty the other (bias, ReLU,
 // mask, BF16 C8 store or FP32 planar store + residual). Before, each CTA took one tile with two
 // stages and did load, MMAs and epilogue in turn, a plane's MMAs at a time: 16 -> 16 channels at
-// 256x256x64 178 us, now 79 (268 MB there and back, 40 us); 48 -> 16 416 us, now 179; 32 -> 32
-// at 128x128x32 66 us, now 37. The tensor pipe is 81% busy then: its M128 K16 MMAs take about
+// 256x256x64 178 us, now 77 (268 MB there and back, 40 us); 48 -> 16 416 us, now 183; 32 -> 32
+// at 128x128x32 66 us, now 38. The tensor pipe is 75% busy then: its M128 K16 MMAs take about
 // 75 cycles for N = 48 and 96, more than their operand reads (44 and 56).
 #include "common.cuh"
 #include "cnn_tc.cuh"

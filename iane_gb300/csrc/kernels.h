@@ -79,7 +79,7 @@ inline bool separable_2d(const DevView& src, const DevView* taps)
 int launch_conv_separable_fast(const DevView& src, const DevView* taps, const DevView& dst, int border,
 	cudaStream_t stream);
 
-// 3-D f32 volumes with TMA-addressable rows, radii r <= 4 (separable_march.cu);
+// 3-D f32 volumes contiguous along x, of any row pitch, radii r <= 4 (separable_march.cu);
 // IANE_GB_UNSUPPORTED without an error when it does not apply.
 int launch_separable_march(const DevView& src, const DevView* taps, const DevView& dst, int border, int r,
 	cudaStream_t stream);

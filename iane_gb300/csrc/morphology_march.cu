@@ -6,19 +6,19 @@
 // back one sample at a time for the x windows, stores and reads those again for the y windows,
 // with two block barriers per plane. Here nothing is shared between warps and nothing is stored
 // before the result:
-//   * a lane owns 4 neighbouring columns and 4 rows of the warp's 128 x 4. The planes come by TMA
-//     into a ring of the warp's own (warp_ring.cuh): no registers are tied up and no block barrier
+//   * a lane owns 4 neighbouring columns and 4 rows of the warp's 128 x 4, or 64 x 8 (ring_narrow).
+//     The planes come by TMA into a ring of the warp's own (warp_ring.cuh): no registers are tied up and no block barrier
 //     is needed;
 //   * the x windows of a row, then the y windows of a column, four at a time, from running
 //     partial extremes (see four_windows);
 //   * along z the 2 R unfinished outputs of every voxel stay in registers: a plane's result
 //     completes the oldest and joins the others.
-// Erosion, zero border, tiled cube kernel -> here: 384 x 384 x 256 3 x 3 x 3 98 -> 51 us, 5 x 5 x 5
-// 131 -> 61 (73% of the measured HBM rate), 7 x 7 x 7 189 -> 81; 512^3 3 x 3 x 3 302 -> 163 us (97%),
-// 5 x 5 x 5 392 -> 190, 7 x 7 x 7 551 -> 262; mirror up to a sixth more. (With the next plane's rows loaded into registers and the
-// neighbours' columns by lane shuffles, two of a warp's 32 lanes without output: 124 us, the loads'
-// latency exposed at three blocks per SM. With a 16-byte cp.async per lane and row: 105 us where it
-// does not spill, the addresses take the registers.)
+// Erosion, zero border, tiled cube kernel -> here: 384 x 384 x 256 3 x 3 x 3 98 -> 53 us, 5 x 5 x 5
+// 131 -> 61 (73% of the measured HBM rate), 7 x 7 x 7 189 -> 83; 512^3 3 x 3 x 3 302 -> 167 us (95%),
+// 5 x 5 x 5 392 -> 190, 7 x 7 x 7 551 -> 265; mirror up to a sixth more. (With the next plane's rows
+// loaded into registers and the neighbours' columns by lane shuffles, two of a warp's 32 lanes without
+// output: 124 us, the loads' latency exposed at three blocks per SM. With a 16-byte cp.async per lane
+// and row: 105 us where it does not spill, the addresses take the registers.)
 //
 // The scan order is the reference's (along each axis increasing for erosion, decreasing for
 // dilation, an update only on a strict compare), so that NaN and signed zeros give its bits. A

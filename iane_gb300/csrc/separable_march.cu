@@ -8,9 +8,9 @@
 // by TMA, or by 4-byte copies where TMA cannot address the rows), filters each row along x, the
 // columns along y, and adds the result to the 2 R unfinished outputs of every voxel along z, all in
 // registers. The y and z sums are packed two columns to an instruction, taps in pairs from shared
-// memory.
-// Mirror border, that kernel -> here: 512^3 3 taps 199 -> 176 us, 5 taps 255 -> 175 (90% of the
-// measured HBM rate), 7 taps 306 -> 246, 9 taps 401 -> 305; 256 x 256 x 64 7 taps 21.6 -> 18.6.
+// memory. A warp is 128 x 4 columns and rows, or 64 x 8 (ring_narrow).
+// Mirror border, that kernel -> here: 512^3 3 taps 199 -> 176 us, 5 taps 255 -> 177 (89% of the
+// measured HBM rate), 7 taps 307 -> 251, 9 taps 401 -> 311; 256 x 256 x 64 7 taps 21.6 -> 18.6.
 // Rows of no multiple of 16 bytes: 253 x 181 x 60 3 taps 32 -> 14.5, 7 taps 63 -> 23, 511 x 401 x 301
 // 7 taps 451 -> 245.
 //
