@@ -43,6 +43,7 @@ namespace {
 constexpr int ROWS_X = 4, ROWS_D = 2;    // rows of the operands
 constexpr int OCT_X = 4, OCT_D = 2;      // and octets
 constexpr int N = OCT_D * ROWS_D * 8;    // 32
+constexpr int MAX_XK = 64;               // voxels of a column along x
 constexpr int STAGES = 6;
 constexpr int THREADS = 192;             // four warps for db and the epilogue, the loader, the MMA issuer
 constexpr int COLS = 512;
@@ -384,7 +385,7 @@ int launch_cnn_wgrad_tc(const uint16_t* x0, int c0, const uint16_t* x1, int c1, 
 	const int jobs = a.groups * co_tiles;
 	// the widest column of those that round the row up least
 	int best = 0;
-	for (int xk = 16; xk <= 64; xk += 16) {
+	for (int xk = 16; xk <= MAX_XK; xk += 16) {
 		const int padded = (w + xk - 1) / xk * xk;
 		if (best == 0 || padded <= best) {
 			best = padded;
@@ -419,9 +420,11 @@ int launch_cnn_wgrad_tc(const uint16_t* x0, int c0, const uint16_t* x1, int c1, 
 	rc = encode_rows_map(&md, dy, co, d, h, w, a.xk, ROWS_D, OCT_D);
 	if (rc) return rc;
 	// a CTA takes the SM's whole TMEM: shared memory enough that no second one lands there
-	const size_t smem = std::max<size_t>(STAGES * stage_bytes(a.xk) + TAIL, 116 * 1024);
+	auto smem_of = [](int xk) { return std::max<size_t>(STAGES * stage_bytes(xk) + TAIL, 116 * 1024); };
+	const size_t smem = smem_of(a.xk);
+	// the most that any width asks for, as other threads may launch between this call and the launch
 	IANE_GB_CUDA(cudaFuncSetAttribute(cnn_wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		static_cast<int>(smem)), "cnn_conv3_wgrad: shared memory attribute");
+		static_cast<int>(smem_of(MAX_XK))), "cnn_conv3_wgrad: shared memory attribute");
 	cnn_wgrad_tc_kernel<<<dim3(a.chunks, a.groups, co_tiles), THREADS, smem, st>>>(m0, m1, md, a);
 	const int n = 27 * co * a.ci + co;
 	wgrad_reduce_kernel<<<(n + 63) / 64, dim3(64, 4), 0, st>>>(partial, a.chunks, co, a.ci, dw, db);

@@ -623,3 +623,36 @@ def test_conv3_weight_gradient_of_unaligned_dy(cuda, shape, c0, c1, co):
     for got, want, mag in zip((dw, db), *wants):
         err = (got.cpu().double() - want).abs()
         assert bool((err <= 1e-5 * mag + 2 ** -22 * want.abs() + 1e-30).all()), float((err - 1e-5 * mag).max())
+
+
+def test_conv3_weight_gradients_of_several_widths_from_several_threads(cuda):
+    # each width has its own shared memory: no thread's launch may find another's limit
+    import threading
+
+    import torch
+
+    failed = []
+
+    def work(width):
+        torch.cuda.set_device(cuda)
+        shape, gen = (2, 4, width), torch.Generator().manual_seed(width)
+        _, x = _act(gen, (16,) + shape)
+        _, dy = _act(gen, (16,) + shape)
+        dw = torch.zeros((16, 16, 27), dtype=torch.float32, device=cuda)
+        scratch = torch.empty(int(_lib().iane_gb_cnn_wgrad_scratch_bytes(16, 0, *shape, 16)), dtype=torch.uint8, device=cuda)
+        stream = torch.cuda.Stream()
+        stream.wait_stream(torch.cuda.default_stream())
+        for _ in range(400):
+            rc = _lib().iane_gb_cnn_conv3_wgrad(_p(x), 16, None, 0, *shape, _p(dy), 16, _p(dw), None, _p(scratch),
+                                                scratch.numel(), stream.cuda_stream)
+            if rc:
+                failed.append((width, rc))
+                break
+        stream.synchronize()
+
+    threads = [threading.Thread(target=work, args=(w,)) for w in (16, 64, 16, 64)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
