@@ -226,8 +226,8 @@ int launch_lanes(const DevView& s, MarchArgs a, cudaStream_t st)
 	const int warps = ring_warps<Ring>(a.in, WARPS);
 	const size_t smem = Ring::bytes(warps);
 	auto kernel = morph_march_kernel<DILATE, R, LANES>;
-	IANE_GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-		"morphology: set shared memory size");
+	IANE_GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Ring::bytes(WARPS))),
+		"morphology: set shared memory size"); // the most, as other threads may launch in between
 	CUtensorMap map{};
 	const int status = ring_map<R, LANES>(&map, s);
 	if (status) return status;

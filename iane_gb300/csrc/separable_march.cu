@@ -168,8 +168,8 @@ int launch_ring(const DevView& s, MarchArgs a, cudaStream_t st)
 	const int warps = ring_warps<Ring>(a.in, WARPS);
 	const size_t smem = Ring::bytes(warps);
 	auto kernel = separable_march_kernel<R, Ring>;
-	IANE_GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-		"separable: set shared memory size");
+	IANE_GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Ring::bytes(WARPS))),
+		"separable: set shared memory size"); // the most, as other threads may launch in between
 	typename Ring::Source source{};
 	if constexpr (std::is_same_v<Ring, WarpRing<R, LANES>>) {
 		const int status = ring_map<R, LANES>(&source, s);

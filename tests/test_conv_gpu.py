@@ -303,6 +303,33 @@ def test_separable_volumes_by_lanes(cuda, shape, taps):
             assert float(np.max(np.abs(to_host(out) - ref) / ref)) <= tol, border
 
 
+def test_separable_volumes_of_several_heights_from_several_threads(cuda):
+    # blocks of one to four warps, each with its own shared memory: no thread's launch may find another's limit
+    import threading
+
+    t = torch()
+    failed = []
+
+    def work(ny):
+        try:
+            t.cuda.set_device(cuda)
+            with t.cuda.stream(t.cuda.Stream()):
+                src = t.rand((6, ny, 64), device="cuda")
+                dst, taps = t.empty_like(src), [t.ones(7, device="cuda")] * 3
+                for _ in range(400):
+                    iane_gb300.convolve_separable(src, taps, dst, "mirror")
+                t.cuda.current_stream().synchronize()
+        except Exception as e:  # noqa: BLE001
+            failed.append((ny, e))
+
+    threads = [threading.Thread(target=work, args=(n,)) for n in (16, 64, 24, 64)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not failed
+
+
 def test_separable_strided_views(cuda):
     t = torch()
     rng = np.random.default_rng(8)
