@@ -187,7 +187,11 @@ __global__ void __launch_bounds__(128, 4) batch_persistent_kernel(const BatchIma
 	const float* tile = reinterpret_cast<const float*>(smem_raw);
 	for (unsigned int n = 0;; ++n) {
 		if (t == 0) take_tile(feed, queues); // the tile after this one
-		if (!mbar_wait_bounded(&sh->full, n & 1)) {
+		const bool landed = mbar_wait_bounded(&sh->full, n & 1);
+		// Thread 0 comes from the queue: apart from its warp, it would sum the tile by itself and the
+		// warp's other lanes after it.
+		__syncwarp();
+		if (!landed) {
 			report_device_status(status, IANE_GB_DEVICE_TIMEOUT);
 			atomicExch(sync.abort, 1);
 			return;

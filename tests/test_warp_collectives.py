@@ -37,3 +37,12 @@ def offences(text):
                          ids=lambda p: p.name)
 def test_warps_are_together_before_a_tensor_memory_load(path):
     assert not list(offences(path.read_text()))
+
+
+def test_the_batch_s_warps_sum_together():
+    # thread 0 takes tiles from the queue while its warp waits for one: brought together before the sums, or
+    # the two parts sum one after the other
+    text = (CSRC / "rl_batch_kernel.cu").read_text()
+    loop = text[text.index("for (unsigned int n = 0;; ++n)"):]
+    wait, sums = loop.index("mbar_wait_bounded(&sh->full"), loop.index("item_sums(tile")
+    assert "__syncwarp();" in loop[wait:sums]
