@@ -305,9 +305,9 @@ int build_graph(iane_gb_rl_batch* b, const DevView* obs, const DevView* est, int
 	}
 	batch_init_kernel<<<dim3(n, kStartBlocks), 256, 0, s0>>>(b->d_init, eps, init);
 	if (iterations > 0) {
-		const BatchQueues queues = make_queues(b->items, b->nx, b->ny, b->order, device_sm_count());
-		st = launch_batch_persistent(b->d_images, b->d_items, queues, 2 * iterations, sync, status,
-			b->blocks_per_sm * device_sm_count(), b->smem, s0);
+		const int sms = device_sm_count(), ctas = b->blocks_per_sm * sms;
+		const BatchQueues queues = make_queues(b->items, b->nx, b->ny, b->order, sms, ctas);
+		st = launch_batch_persistent(b->d_images, b->d_items, queues, 2 * iterations, sync, status, ctas, b->smem, s0);
 		if (st) return abort_capture(st);
 	} else {
 		batch_init_kernel<<<dim3(n, kStartBlocks), 256, 0, s0>>>(b->d_init, eps, -1);
@@ -408,7 +408,7 @@ int autotune(iane_gb_rl_batch* b, cudaStream_t stream)
 		if (cudaMemcpy(d_items, items.data(), items.size() * sizeof(BatchItem), cudaMemcpyHostToDevice) != cudaSuccess) {
 			return cuda_fail(cudaGetLastError(), "autotune: upload items");
 		}
-		const BatchQueues queues = make_queues(items, b->nx, b->ny, order, sms);
+		const BatchQueues queues = make_queues(items, b->nx, b->ny, order, sms, bps * sms);
 		ms = 0.0f;
 		for (int rep = 0; rep < 3; ++rep) {
 			if (cudaMemsetAsync(sync.queue, 0, sync_bytes(n), stream) != cudaSuccess) {

@@ -164,7 +164,9 @@ __device__ __forceinline__ void issue_tile(const FeedArgs& a)
 // that tile is still landing, its loads (tile, taps, descriptor, all asynchronous) start as soon
 // as the sums have read the buffers and land during the epilogue. A tile in hand never waits for
 // its image before the tile in work is counted done, so the earliest unfinished tile can always
-// proceed. Each warp counts itself done: no barrier follows the epilogue.
+// proceed. Each warp counts itself done: no barrier follows the epilogue. Where a phase has few tiles
+// for each CTA (batch_ahead), a CTA takes the next item only then: in its hand the item would wait for
+// it, and there are idle ones.
 __global__ void __launch_bounds__(128, 4) batch_persistent_kernel(const BatchImage* __restrict__ images,
 	const BatchItem* __restrict__ items, const __grid_constant__ BatchQueues queues, int phases, BatchSync sync,
 	int* status, unsigned int stage)
@@ -186,7 +188,11 @@ __global__ void __launch_bounds__(128, 4) batch_persistent_kernel(const BatchIma
 	if (t == 0) issue_tile(feed);
 	const float* tile = reinterpret_cast<const float*>(smem_raw);
 	for (unsigned int n = 0;; ++n) {
-		if (t == 0) take_tile(feed, queues); // the tile after this one
+		bool held = false; // thread 0: the tile after this one is in hand
+		if (t == 0 && (queues.ahead || (sh->phase >= 0 && sh->next + 1 < sh->item.count))) {
+			take_tile(feed, queues);
+			held = true;
+		}
 		const bool landed = mbar_wait_bounded(&sh->full, n & 1);
 		// Thread 0 comes from the queue: apart from its warp, it would sum the tile by itself and the
 		// warp's other lanes after it.
@@ -213,7 +219,8 @@ __global__ void __launch_bounds__(128, 4) batch_persistent_kernel(const BatchIma
 		__syncthreads(); // tile and taps have been read
 		bool waiting = false;
 		if (t == 0) {
-			waiting = sh->phase > 0 && !counter_reached(load_acquire(sync.done + sh->item.image), tile_need(*sh));
+			waiting = !held ||
+				(sh->phase > 0 && !counter_reached(load_acquire(sync.done + sh->item.image), tile_need(*sh)));
 			if (!waiting) issue_tile(feed);
 		}
 		const int xo = wx + kRX * (lane & 3), yo = wy + kRY * (lane >> 2);
@@ -235,8 +242,9 @@ __global__ void __launch_bounds__(128, 4) batch_persistent_kernel(const BatchIma
 			atomicAdd(&sync.done[m.y], 1u);
 		}
 		if (waiting) {
+			if (!held) take_tile(feed, queues);
 			// bounded: a wait that gives up aborts the run
-			if (!wait_counter(sync.done + sh->item.image, tile_need(*sh), sync.abort, status)) sh->phase = -1;
+			if (sh->phase > 0 && !wait_counter(sync.done + sh->item.image, tile_need(*sh), sync.abort, status)) sh->phase = -1;
 			issue_tile(feed);
 		}
 	}

@@ -32,7 +32,7 @@ extern "C" int queues(const int* nx, const int* ny, const int* kx, const int* ky
 {
 	const auto list_nx = list(nx, n), list_ny = list(ny, n);
 	const auto made = make_items(list_nx, list_ny, list(kx, n), list(ky, n), order, group);
-	const BatchQueues q = make_queues(made, list_nx, list_ny, order, sms);
+	const BatchQueues q = make_queues(made, list_nx, list_ny, order, sms, sms);
 	for (const BatchItem& i : made) {
 		const int v[] = {i.image, i.x0, i.y0, i.count, i.image_tiles, i.kx, i.ky};
 		std::memcpy(items, v, sizeof v);
@@ -123,8 +123,9 @@ def test_items_cover_the_batch_and_queues_share_the_sms(plan, n, sms, order, gro
             assert start.count(c) <= max(1.0, work[c] / sum(work) * sms + 1)
 
 
-def simulate(plan, images, order, group, sms, ctas_per_sm, phases, rng):
-    """One run: every CTA has a tile in work and the next one in hand, as in batch_persistent_kernel."""
+def simulate(plan, images, order, group, sms, ctas_per_sm, phases, ahead, rng):
+    """One run: every CTA has a tile in work and, with `ahead` or within an item, the next one in hand, as in
+    batch_persistent_kernel."""
     items, queues, start = queues_of(plan, images, order, group, sms)
     heads, done, true_done = [0] * len(queues), [0] * len(images), {}
     finished = set()
@@ -167,9 +168,11 @@ def simulate(plan, images, order, group, sms, ctas_per_sm, phases, rng):
         tile = issue(cta)
         while tile is not None:
             yield rng.uniform(0.0, 1.0)
-            take(cta)
+            held = ahead or cta["next"] + 1 < cta["item"][3]
+            if held:
+                take(cta)
             yield rng.uniform(0.5, 3.0)  # landing and sums
-            later, issued = not free(cta), False
+            later, issued = not held or not free(cta), False
             if not later:
                 tile_after, issued = issue(cta), True
             for _ in range(4):  # the warps' epilogues, each counting for itself
@@ -179,6 +182,8 @@ def simulate(plan, images, order, group, sms, ctas_per_sm, phases, rng):
             assert tile[:4] not in finished
             finished.add(tile[:4])
             if not issued:
+                if not held:
+                    take(cta)
                 while not free(cta):
                     yield None
                 tile_after = issue(cta)
@@ -212,10 +217,11 @@ def simulate(plan, images, order, group, sms, ctas_per_sm, phases, rng):
 
 @pytest.mark.parametrize("group", [0, 2, 3])
 @pytest.mark.parametrize("order", [0, 1])
+@pytest.mark.parametrize("ahead", [False, True])
 @pytest.mark.parametrize("sms,ctas_per_sm", [(1, 1), (2, 1), (3, 4), (40, 2)])
-def test_tiles_in_work_and_in_hand_keep_the_order_and_end(plan, sms, ctas_per_sm, order, group):
+def test_tiles_in_work_and_in_hand_keep_the_order_and_end(plan, sms, ctas_per_sm, ahead, order, group):
     for seed in range(4):
         rng = random.Random(seed * 100 + sms)
         images = [(64 * rng.randint(1, 9), 64 * rng.randint(1, 3), rng.choice([1, 5, 5, 7, 15, 31]), 5)
                   for _ in range(rng.randint(1, 6))]
-        simulate(plan, images, order, group, sms, ctas_per_sm, 6, rng)
+        simulate(plan, images, order, group, sms, ctas_per_sm, 6, ahead, rng)
